@@ -294,15 +294,11 @@ int gb_bh_export(gb_bh_t *h, int what, void *dst, void *stream);
 
 int gb_bh_diag(gb_bh_t *h, gb_diag_t *out, int reset);
 
-/* Traversal shape.  1 and 2: warp-coherent, the warp's 32 (or 64, two per
- * lane) key-consecutive targets walk the tree together, one node record per
- * warp step.  0: per lane, each lane walks its own target with its own
- * stack (max_stack <= 127 and n <= 2^25 + 1; otherwise mode 1 runs).  -1
- * (default): 0 below n = 131,072, 1 from there.  All modes give
- * bit-identical results: each target meets its nodes in the same order.
- * Mode 1 is fastest on the 1M disk (per-lane record loads diverge); mode 0
- * on small systems, where a warp-coherent launch has too few warps to hide
- * each step's latency.
+/* Traversal shape.  -1 (default), 0, 1 and 2: the per-particle walk, in which
+ * each target accepts exactly the reference's node set (4 to 32
+ * key-consecutive targets share a warp, by n).  The four values run the same
+ * kernel and give bit-identical results; 0 to 2 named kernels of their own
+ * once and stay accepted.
  * 3 (opt-in): group walk.  The targets are cut into groups, the largest
  * subtrees with at most 32 leaves; a group accepts a node when
  * size^2 < theta^2 (dmin^2 + eps^2), dmin the distance from the node's

@@ -18,14 +18,13 @@
 //               reads): no floating-point atomics, and the result is
 //               independent of scheduling (:124-177 use FP64 atomics on
 //               every ancestor instead)
-//   6 traverse  warp-coherent walk: 32 key-consecutive targets share one
-//               shared-memory stack of (node, lane mask); every lane applies
-//               the reference's own acceptance test size^2 < theta^2 (r^2 +
-//               eps^2) (:204-210), so each particle accepts exactly the node
-//               set of _traverse (:180-217); a per-lane count reproduces the
-//               max_stack rule (:212) and the skipped pushes are counted
-//               instead of being lost silently.  Closing kick fused in the
-//               epilogue for KDK steps.
+//   6 traverse  per-particle walk: 4 to 32 key-consecutive targets share a
+//               warp and its list of opened nodes; every target applies the reference's own acceptance
+//               test size^2 < theta^2 (r^2 + eps^2) (:204-210), so each
+//               particle accepts exactly the node set of _traverse
+//               (:180-217); the max_stack rule (:212) is kept and the skipped
+//               pushes are counted instead of being lost silently.  Closing
+//               kick fused in the epilogue for KDK steps.
 #include <algorithm>
 #include <cstdio>
 
@@ -479,7 +478,7 @@ struct gb_bh {
     cudaEvent_t ev[GB_BH_TIMING_STEPS * (GB_BH_STAGES + 1)];
     uint64_t launches;  // kernels launched by this handle (host count)
     int pending_slot;   // timing slot of the last gb_bh_build
-    int tpl;            // traversal shape: -1 by n (default), 0 per lane, 1 or 2 targets per lane
+    int tpl;            // traversal shape: -1 .. 2 the particle walk, 3 the group walk
     // One KDK step captured as a CUDA graph (gb_bh_kdk), replayed per step
     // on the handle's own stream and joined to the caller's by events.
     // gexec[0]: a plain step; gexec[1]: a step that also writes the tree
@@ -546,23 +545,6 @@ extern "C" int gb_bh_create(gb_bh_t **out, int64_t n_max, int key_bits) {
     h->key_bits = key_bits;
     h->tpl = -1;
     h->use_graph = 1;
-    {
-        const int smem_max = (int)sizeof(int) * LANE_MAX_STACK * LANE_THREADS;
-        const void *lk[] = {(const void *)bh_traverse_lane_kernel<false, false, false>,
-                            (const void *)bh_traverse_lane_kernel<false, true, false>,
-                            (const void *)bh_traverse_lane_kernel<true, false, false>,
-                            (const void *)bh_traverse_lane_kernel<true, true, false>,
-                            (const void *)bh_traverse_lane_kernel<false, false, true>,
-                            (const void *)bh_traverse_lane_kernel<false, true, true>,
-                            (const void *)bh_traverse_lane_kernel<true, false, true>,
-                            (const void *)bh_traverse_lane_kernel<true, true, true>};
-        for (const void *f : lk) {
-            if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max) != cudaSuccess) {
-                delete h;
-                return fail(GB_ECUDA, "gb_bh_create: cannot enable %d bytes of shared memory", smem_max);
-            }
-        }
-    }
     h->n = -1;
     h->cur = 0;
     const int64_t nn = n_max, ni = std::max<int64_t>(n_max - 1, 1), nodes = 2 * n_max;
@@ -675,19 +657,6 @@ static int check_ptr(const void *p, const char *name) {
     return GB_OK;
 }
 
-template <bool KDK, bool COUNT, bool PHI>
-static void launch_lane(unsigned grid, size_t smem, const TravArgs &a, float *phi, const int *parent, int2 r,
-                        cudaStream_t s) {
-    bh_traverse_lane_kernel<KDK, COUNT, PHI><<<grid, LANE_THREADS, smem, s>>>(a, phi, parent, r.x, r.y);
-}
-
-template <bool KDK, bool COUNT, bool PHI>
-static void launch_warp(int tpl, unsigned grid, const TravArgs &a, float *phi, const int *parent, int2 r,
-                        cudaStream_t s) {
-    if (tpl == 2) bh_traverse_kernel<KDK, COUNT, 2, PHI><<<grid, TRAV_WARPS * 32, 0, s>>>(a, phi, parent, r.x, r.y);
-    else bh_traverse_kernel<KDK, COUNT, 1, PHI><<<grid, TRAV_WARPS * 32, 0, s>>>(a, phi, parent, r.x, r.y);
-}
-
 // Dispatches L<KDK, COUNT, PHI>::go(args...) on run-time flags.
 template <template <bool, bool, bool> class L, typename... Args>
 static void dispatch3(bool kdk, bool count, bool phi, Args... args) {
@@ -704,23 +673,24 @@ static void dispatch3(bool kdk, bool count, bool phi, Args... args) {
     }
 }
 template <bool KDK, bool COUNT, bool PHI>
-struct LaneLaunch {
-    static void go(unsigned grid, size_t smem, const TravArgs *a, float *phi, const int *parent, int2 r,
-                   cudaStream_t s) {
-        launch_lane<KDK, COUNT, PHI>(grid, smem, *a, phi, parent, r, s);
-    }
-};
-template <bool KDK, bool COUNT, bool PHI>
 struct GroupLaunch {
     static void go(unsigned grid, const TravArgs *a, const int *gsize, float *phi, int2 r, cudaStream_t s) {
         bh_group_kernel<KDK, COUNT, PHI><<<grid, GW_WARPS * 32, 0, s>>>(*a, gsize, phi, r.x, r.y);
     }
 };
 template <bool KDK, bool COUNT, bool PHI>
-struct WarpLaunch {
-    static void go(int tpl, unsigned grid, const TravArgs *a, float *phi, const int *parent, int2 r,
-                   cudaStream_t s) {
-        launch_warp<KDK, COUNT, PHI>(tpl, grid, *a, phi, parent, r, s);
+struct WalkLaunch {
+    template <int T>
+    static void run(int2 r, const TravArgs *a, float *phi, cudaStream_t s) {
+        const int64_t groups = ((int64_t)r.y - r.x + T - 1) / T;
+        bh_walk_kernel<KDK, COUNT, PHI, T><<<(unsigned)((groups + WALK_WARPS - 1) / WALK_WARPS), WALK_WARPS * 32,
+                                             WALK_WARPS * sizeof(WalkWarp<T>), s>>>(*a, phi, r.x, r.y);
+    }
+    static void go(int group, int2 r, const TravArgs *a, float *phi, cudaStream_t s) {
+        if (group == 4) run<4>(r, a, phi, s);
+        else if (group == 8) run<8>(r, a, phi, s);
+        else if (group == 16) run<16>(r, a, phi, s);
+        else run<32>(r, a, phi, s);
     }
 };
 
@@ -754,11 +724,7 @@ static int traverse(gb_bh_t *h, float4 *acc, float4 *vel, float *phi, float thet
     a.diag = h->diag;
     a.pot = pot;
     const bool count = (flags & GB_COUNT_WORK) != 0;
-    // By n: per-lane walks below LANE_AUTO_N, where a warp-coherent launch
-    // has too few warps to hide each step's latency (1M disk: 3.44 ms
-    // warp-coherent against 5.84 ms per lane; 10k: 0.24 against 0.18 ms).
-    const int shape = h->tpl >= 0 ? h->tpl : (n < LANE_AUTO_N ? 0 : 1);
-    if (shape == 3) {
+    if (h->tpl == 3) {
         const int64_t warps = (nt + 31) / 32;
         const unsigned grid = (unsigned)((warps + GW_WARPS - 1) / GW_WARPS);
         if (h->groups_n != n) {
@@ -779,15 +745,9 @@ static int traverse(gb_bh_t *h, float4 *acc, float4 *vel, float *phi, float thet
             h->groups_n = n;
         }
         dispatch3<GroupLaunch>(kdk, count, phi != nullptr, grid, &a, (const int *)h->gsize, phi, range, s);
-    } else if (shape == 0 && max_stack <= LANE_MAX_STACK && n - 1 <= ((int64_t)1 << LANE_KBITS)) {
-        const unsigned grid = (unsigned)((nt + LANE_THREADS - 1) / LANE_THREADS);
-        const size_t smem = sizeof(int) * (size_t)std::max(max_stack, 1) * LANE_THREADS;
-        dispatch3<LaneLaunch>(kdk, count, phi != nullptr, grid, smem, &a, phi, (const int *)h->parent, range, s);
     } else {
-        const int tpl = shape == 2 ? 2 : 1;
-        const int64_t warps = (nt + 32 * tpl - 1) / (32 * tpl);
-        const unsigned grid = (unsigned)((warps + TRAV_WARPS - 1) / TRAV_WARPS);
-        dispatch3<WarpLaunch>(kdk, count, phi != nullptr, tpl, grid, &a, phi, (const int *)h->parent, range, s);
+        const int group = n < WALK_4_N ? 4 : n < WALK_8_N ? 8 : n < WALK_16_N ? 16 : 32;
+        dispatch3<WalkLaunch>(kdk, count, phi != nullptr, group, range, &a, phi, s);
     }
     GB_CUDA_TRY(cudaGetLastError());
     mark(h, slot, 5, s);

@@ -1,14 +1,11 @@
 // Tree traversal kernels of the LBVH Barnes-Hut path (included by gb_bh.cu,
 // which builds the tree they walk):
-//   bh_traverse_kernel       warp-coherent walk: 32 (or 64) key-consecutive
-//                            targets share one shared-memory stack of (node,
-//                            lane mask); every lane applies the reference's
-//                            own acceptance test (core/solvers/barnes_hut.py:
-//                            204-210), so each particle accepts exactly the
-//                            node set of _traverse (:180-217)
-//   bh_traverse_lane_kernel  the same walk with one stack per lane
-//   bh_group_kernel          the opt-in group walk (a refinement of each
-//                            target's node set, one walk per leaf group)
+//   bh_walk_kernel   the per-particle walk (traversal shapes -1, 0, 1, 2):
+//                    each particle accepts exactly the node set of the
+//                    reference's _traverse (core/solvers/barnes_hut.py:
+//                    180-217)
+//   bh_group_kernel  the opt-in group walk (a refinement of each target's
+//                    node set, one walk per leaf group)
 // Node records: inode[3k .. 3k+2] = the two children of internal node k as
 // (left, right) pairs {x, y, z, m, size^2, id}; root[0..1] = the root's.
 #pragma once
@@ -16,9 +13,6 @@
 #include "gb_common.cuh"
 
 namespace gb {
-
-constexpr int TRAV_WARPS = 4;
-constexpr int TRAV_STACK = 128;  // > maximum Karras depth (63 + 31 levels)
 
 // --------------------------------------------------------------- traverse
 struct TravArgs {
@@ -36,441 +30,13 @@ struct TravArgs {
     ExtPot pot;  // analytic potential added in the epilogue (pot.on)
 };
 
-struct Lane {
-    float px, py, pz, ax, ay, az;
-    f2 PX, PY, PZ;  // (p, p) pairs
-    f2 AX, AY, AZ;  // accumulators for (left, right) children
-    unsigned n_int, n_test, drops;
-};
-
-// Tree-potential sums of a lane (PHI kernels only): pw for the root, PW for
-// the (left, right) children.  The children's terms are added as sc * r2
-// (= m / |d| up to rsqrt rounding) from the masked force factor, the lane's
-// own leaf included; self records whether the walk reached it (its parent,
-// internal node kp, was expanded for the lane), and the epilogue then
-// removes its term m rsqrt(eps^2)^3 eps^2.
-struct LanePhi {
-    float pw, pm;
-    f2 PW;
-    int kp;
-    bool self;
-};
-
-// The lane's potential sum without its own leaf's term.
-__device__ __forceinline__ float lane_phi(const LanePhi &W, float eps2) {
-    float wl, wr;
-    unpack2(W.PW, wl, wr);
-    const float pw = W.pw + (wl + wr);
-    if (!W.self) return pw;
-    const float inv = rsqrt_approx(eps2);
-    return __fmaf_rn(-((W.pm * inv) * (inv * inv)), eps2, pw);
-}
-
-// One child for one lane of the expanding mask (branch-free).  Leaves carry
-// size2 = -1 in the record, so the one comparison size2 < theta^2 (|d|^2 +
-// eps^2) accepts every leaf and applies the reference's test (:208) to
-// internal nodes.  An accepted child adds its monopole; the lane's own leaf
-// (which the reference skips, :198) sits exactly at the lane's position, so
-// its term is d * (...) = +0 and needs no test.  A rejected (internal) child
-// is opened.  Returns "open".  PHI: an accepted child other than the lane's
-// own leaf also adds its monopole potential m / |d| (|d|^2 = d.d + eps^2),
-// the tree form of the potential_energy sum (core/solvers/gravity.py:47-55).
-template <bool COUNT, bool PHI>
-__device__ __forceinline__ bool visit_child(Lane &L, LanePhi &W, const TravArgs &a, float4 q, float size2, int id,
-                                            int s, bool in) {
-    const float dx = q.x - L.px, dy = q.y - L.py, dz = q.z - L.pz;
-    const float r2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmaf_rn(dx, dx, a.eps2)));
-    const bool accept = size2 < a.theta2 * r2;
-    const bool add = in && accept;
-    const float inv = rsqrt_approx(r2);
-    const float sc = add ? q.w * inv * inv * inv : 0.f;
-    L.ax = __fmaf_rn(sc, dx, L.ax);
-    L.ay = __fmaf_rn(sc, dy, L.ay);
-    L.az = __fmaf_rn(sc, dz, L.az);
-    if (PHI) W.pw += (add && id != s) ? q.w * inv : 0.f;  // the root: never the own leaf
-    if (COUNT) {
-        L.n_int += (add && id != s) ? 1u : 0u;
-        L.n_test += (in && size2 >= 0.f) ? 1u : 0u;
-    }
-    return in && !accept;
-}
-
-// Both children of an expanded node for one lane, on packed (left, right)
-// pairs: the same test and monopole as visit_child, two children per
-// instruction.  Sets openL / openR.  PHI as in visit_child.
-template <bool COUNT, bool PHI>
-__device__ __forceinline__ void visit_pair(Lane &L, LanePhi &W, const TravArgs &a, ulonglong2 A, ulonglong2 B,
-                                           float4 C, int s, bool in, f2 E2, f2 TH2, bool &openL, bool &openR) {
-    const f2 dx = sub2(A.x, L.PX), dy = sub2(A.y, L.PY), dz = sub2(B.x, L.PZ);
-    f2 r2 = fma2(dx, dx, E2);
-    r2 = fma2(dy, dy, r2);
-    r2 = fma2(dz, dz, r2);
-    const f2 t = mul2(TH2, r2);
-    float r2L, r2R, tL, tR;
-    unpack2(r2, r2L, r2R);
-    unpack2(t, tL, tR);
-    const bool accL = C.x < tL, accR = C.y < tR;
-    const f2 inv = pack2(rsqrt_approx(r2L), rsqrt_approx(r2R));
-    const f2 sc = mul2(mul2(B.y, inv), mul2(inv, inv));
-    float scL, scR;
-    unpack2(sc, scL, scR);
-    const f2 scm = pack2((in && accL) ? scL : 0.f, (in && accR) ? scR : 0.f);
-    L.AX = fma2(scm, dx, L.AX);
-    L.AY = fma2(scm, dy, L.AY);
-    L.AZ = fma2(scm, dz, L.AZ);
-    if (PHI) W.PW = fma2(scm, r2, W.PW);
-    if (COUNT) {
-        L.n_int += (in && accL && __float_as_int(C.z) != s) ? 1u : 0u;
-        L.n_int += (in && accR && __float_as_int(C.w) != s) ? 1u : 0u;
-        L.n_test += (in && C.x >= 0.f) ? 1u : 0u;
-        L.n_test += (in && C.y >= 0.f) ? 1u : 0u;
-    }
-    openL = in && !accL;
-    openR = in && !accR;
-}
-
-// The reference's push rule (:212): a lane that opens a node popped at stack
-// depth sp pushes its children only if sp + 2 <= max_stack.  sp is uniform
-// over the warp, so the (rare) drop path is a uniform branch.
-__device__ __forceinline__ bool apply_room(Lane &L, bool open, int sp, int max_stack) {
-    if (sp + 2 <= max_stack) return open;
-    L.drops += open ? 1u : 0u;
-    return false;
-}
-
-// Warp-coherent traversal: TPL x 32 key-consecutive targets per warp walk the
-// tree together (TPL targets per lane: slot q of lane l is target wbase +
-// 32 q + l).  The warp expands one internal node per iteration: it loads the
-// node's two-children record (48 B) and every lane visits both children for
-// each of its slots in the node's masks (right first, as the reference pops
-// it first).  The right child, if any slot opened it, is expanded next
-// straight from registers; an opened left child waits on a shared-memory
-// stack of {node, mask slot 0, mask slot 1, sp}.  sp, the depth of the
-// reference's per-particle stack when a node is popped, depends only on the
-// node's path (one pending left sibling per right turn), so it travels with
-// the node.
-// PHI: phi receives the tree potential sum of every particle (no G).  It is
-// a kernel argument of its own: inside TravArgs it changed the register
-// allocation of the kernels without it (46 against 48 registers, 13% more
-// instructions per node expansion, measured).
-template <bool KDK, bool COUNT, int TPL, bool PHI>
-__global__ void __launch_bounds__(TRAV_WARPS * 32)
-bh_traverse_kernel(TravArgs a, float *__restrict__ phi, const int *__restrict__ parent, int s0, int s1) {
-    __shared__ int4 stk[TRAV_WARPS][TRAV_STACK];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int wbase = s0 + (blockIdx.x * TRAV_WARPS + wid) * (32 * TPL);
-    if (wbase >= s1) return;  // whole warp out of range
-    const int n = a.n;
-    int s[TPL];
-    bool valid[TPL];
-    Lane L[TPL];
-    LanePhi W[TPL];
-#pragma unroll
-    for (int q = 0; q < TPL; ++q) {
-        s[q] = wbase + 32 * q + lane;
-        valid[q] = s[q] < s1;
-        L[q].px = L[q].py = L[q].pz = 0.f;
-        W[q].pm = 0.f;
-        if (valid[q]) {
-            const float4 p = __ldg(a.leaf + s[q]);
-            L[q].px = p.x; L[q].py = p.y; L[q].pz = p.z;
-            W[q].pm = p.w;
-        }
-        L[q].ax = L[q].ay = L[q].az = 0.f;
-        L[q].PX = pack2(L[q].px, L[q].px);
-        L[q].PY = pack2(L[q].py, L[q].py);
-        L[q].PZ = pack2(L[q].pz, L[q].pz);
-        L[q].AX = L[q].AY = L[q].AZ = 0ull;
-        W[q].pw = 0.f;
-        W[q].PW = 0ull;
-        W[q].self = false;
-        W[q].kp = (PHI && valid[q] && n >= 2) ? __ldg(parent + s[q]) - n : -1;
-        L[q].n_int = L[q].n_test = L[q].drops = 0;
-    }
-    const f2 E2 = pack2(a.eps2, a.eps2), TH2 = pack2(a.theta2, a.theta2);
-    unsigned overflow = 0, bad = 0, iters = 0;
-    int top = 0;
-    int k = 0, sp = 0;
-    unsigned m[TPL];
-    unsigned any = 0;
-#pragma unroll
-    for (int q = 0; q < TPL; ++q) m[q] = 0;
-    if (n >= 2) {
-        // The root is popped first, with an empty stack (sp = 0).
-        const float4 R0 = __ldg(a.root), R1 = __ldg(a.root + 1);
-#pragma unroll
-        for (int q = 0; q < TPL; ++q) {
-            const bool want = apply_room(L[q], visit_child<COUNT, PHI>(L[q], W[q], a, R0, R1.x, n, s[q], valid[q]),
-                                         0, a.max_stack);
-            m[q] = __ballot_sync(0xffffffffu, want);
-            any |= m[q];
-        }
-    }
-    while (any) {
-        if ((unsigned)k >= (unsigned)(n - 1)) {  // never for a consistent tree
-#pragma unroll
-            for (int q = 0; q < TPL; ++q) bad += ((m[q] >> lane) & 1u);
-            any = 0;
-        } else {
-            const ulonglong2 A = __ldg(reinterpret_cast<const ulonglong2 *>(a.inode + 3 * k));
-            const ulonglong2 B = __ldg(reinterpret_cast<const ulonglong2 *>(a.inode + 3 * k + 1));
-            const float4 C = __ldg(a.inode + 3 * k + 2);
-            const int idL = __float_as_int(C.z), idR = __float_as_int(C.w);
-            if (COUNT) ++iters;
-            unsigned omL[TPL], omR[TPL], anyL = 0, anyR = 0;
-            // Room for both children's pushes (the right child is popped at
-            // depth sp + 1): one warp-uniform test; the per-child rule only
-            // runs near max_stack.
-            const bool room2 = sp + 3 <= a.max_stack;
-#pragma unroll
-            for (int q = 0; q < TPL; ++q) {
-                const bool in = (m[q] >> lane) & 1u;
-                bool wantR, wantL;
-                visit_pair<COUNT, PHI>(L[q], W[q], a, A, B, C, s[q], in, E2, TH2, wantL, wantR);
-                if (PHI) W[q].self |= in && k == W[q].kp;
-                if (!room2) {
-                    wantR = apply_room(L[q], wantR, sp + 1, a.max_stack);
-                    wantL = apply_room(L[q], wantL, sp, a.max_stack);
-                }
-                omL[q] = __ballot_sync(0xffffffffu, wantL);
-                omR[q] = __ballot_sync(0xffffffffu, wantR);
-                anyL |= omL[q];
-                anyR |= omR[q];
-            }
-            if (anyR) {  // expand the right child next; a left child waits on the stack
-                if (anyL) {
-                    if (top < TRAV_STACK) {
-                        // Every lane stores the same entry (no lane predicate).
-                        stk[wid][top] = make_int4(idL - n, (int)omL[0], TPL > 1 ? (int)omL[TPL - 1] : 0, sp);
-                        ++top;
-                    } else {
-#pragma unroll
-                        for (int q = 0; q < TPL; ++q) overflow += ((omL[q] >> lane) & 1u);
-                    }
-                }
-                k = idR - n;
-#pragma unroll
-                for (int q = 0; q < TPL; ++q) m[q] = omR[q];
-                sp = sp + 1;
-                continue;
-            }
-            if (anyL) {  // only the left child was opened: expand it next directly
-                k = idL - n;
-#pragma unroll
-                for (int q = 0; q < TPL; ++q) m[q] = omL[q];
-                continue;
-            }
-            any = 0;
-        }
-        if (top > 0) {
-            __syncwarp();
-            const int4 e = stk[wid][--top];
-            k = e.x;
-            m[0] = (unsigned)e.y;
-            if (TPL > 1) m[TPL - 1] = (unsigned)e.z;
-            sp = e.w;
-            any = m[0] | m[TPL - 1];
-            __syncwarp();
-        }
-    }
-    // Counters: one atomic per warp and counter.
-    unsigned dsum = 0, osum = overflow, bsum = bad;
-#pragma unroll
-    for (int q = 0; q < TPL; ++q) dsum += L[q].drops;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        dsum += __shfl_xor_sync(0xffffffffu, dsum, o);
-        osum += __shfl_xor_sync(0xffffffffu, osum, o);
-        bsum += __shfl_xor_sync(0xffffffffu, bsum, o);
-    }
-    if (COUNT) {
-        unsigned isum = 0, tsum = 0;
-#pragma unroll
-        for (int q = 0; q < TPL; ++q) {
-            isum += L[q].n_int;
-            tsum += L[q].n_test;
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            isum += __shfl_xor_sync(0xffffffffu, isum, o);
-            tsum += __shfl_xor_sync(0xffffffffu, tsum, o);
-        }
-        if (lane == 0) {
-            atomicAdd(a.diag + DIAG_NODE_READS, (unsigned long long)iters);
-            atomicAdd(a.diag + DIAG_ROOT_READS, 1ull);
-            atomicAdd(a.diag + DIAG_INTERACTIONS, (unsigned long long)isum);
-            atomicAdd(a.diag + DIAG_TESTS, (unsigned long long)tsum);
-        }
-    }
-    if (lane == 0) {
-        if (dsum) atomicAdd(a.diag + DIAG_STACK_DROPS, (unsigned long long)dsum);
-        if (osum) atomicAdd(a.diag + DIAG_STACK_OVERFLOW, (unsigned long long)osum);
-        if (bsum) atomicAdd(a.diag + DIAG_BAD_TREE, (unsigned long long)bsum);
-    }
-    // Epilogue: scatter to the original particle index.
-#pragma unroll
-    for (int q = 0; q < TPL; ++q) {
-        if (!valid[q]) continue;
-        const uint32_t p = __ldg(a.order + s[q]);
-        if (p >= (uint32_t)n) continue;
-        float xl, xr, yl, yr, zl, zr;
-        unpack2(L[q].AX, xl, xr);
-        unpack2(L[q].AY, yl, yr);
-        unpack2(L[q].AZ, zl, zr);
-        float gx = a.G * (L[q].ax + (xl + xr)), gy = a.G * (L[q].ay + (yl + yr)),
-              gz = a.G * (L[q].az + (zl + zr));
-        if (a.pot.on) ext_acc_add(a.pot, L[q].px, L[q].py, L[q].pz, gx, gy, gz);
-        if (PHI) phi[p] = lane_phi(W[q], a.eps2);
-        if (KDK) {
-            const float4 vh = a.vel[p];
-            a.vel[p] = make_float4(kick(vh.x, gx, a.h), kick(vh.y, gy, a.h), kick(vh.z, gz, a.h), vh.w);
-            a.acc[p] = make_float4(gx, gy, gz, 0.f);
-        } else if (a.accumulate) {
-            float4 o = a.acc[p];
-            o.x += gx; o.y += gy; o.z += gz;
-            a.acc[p] = o;
-        } else {
-            a.acc[p] = make_float4(gx, gy, gz, 0.f);
-        }
-    }
-}
-
-// Per-lane traversal: each lane walks the tree for its own target, exactly
-// the reference's per-particle loop (:185-217) on the two-children records:
-// expanding node k tests both children (the reference pushes both and then
-// tests each when popped; the decisions do not depend on when a child is
-// tested), continues into an opened right child directly (the reference pops
-// the right child first) and keeps an opened left child on the lane's own
-// shared-memory stack.  Lanes of a warp are at different nodes, so a warp
-// runs as many iterations as its busiest lane, instead of the union of all
-// its lanes' nodes as the warp-coherent kernel does.  Stack entries hold
-// the internal index (25 bits) and the reference's stack depth d when the
-// node is popped (7 bits): a right child is popped at d + 1 and a left child
-// at d, which gives the max_stack rule exactly.  Layout [depth][thread]:
-// every lane hits its own bank whatever its depth.
-constexpr int LANE_THREADS = 128;
-constexpr int LANE_KBITS = 25;
-constexpr int LANE_MAX_STACK = 127;
-// Below this n the traversal runs per lane by default (measured crossover
-// between 100k and 300k particles on a disk).
-constexpr int64_t LANE_AUTO_N = 131072;
-
-template <bool KDK, bool COUNT, bool PHI>
-__global__ void __launch_bounds__(LANE_THREADS)
-bh_traverse_lane_kernel(TravArgs a, float *__restrict__ phi, const int *__restrict__ parent, int s0, int s1) {
-    extern __shared__ int lstk[];  // [max_stack][LANE_THREADS]
-    const int tid = threadIdx.x;
-    const int n = a.n;
-    const int s = s0 + blockIdx.x * LANE_THREADS + tid;
-    const bool valid = s < s1;
-    Lane L;
-    LanePhi W;
-    W.pw = 0.f;
-    W.PW = 0ull;
-    W.pm = 0.f;
-    W.self = false;
-    W.kp = (PHI && valid && n >= 2) ? __ldg(parent + s) - n : -1;
-    L.px = L.py = L.pz = 0.f;
-    if (valid) {
-        const float4 p = __ldg(a.leaf + s);
-        L.px = p.x; L.py = p.y; L.pz = p.z;
-        W.pm = p.w;
-    }
-    L.ax = L.ay = L.az = 0.f;
-    L.PX = pack2(L.px, L.px);
-    L.PY = pack2(L.py, L.py);
-    L.PZ = pack2(L.pz, L.pz);
-    L.AX = L.AY = L.AZ = 0ull;
-    L.n_int = L.n_test = L.drops = 0;
-    const f2 E2 = pack2(a.eps2, a.eps2), TH2 = pack2(a.theta2, a.theta2);
-    unsigned overflow = 0, bad = 0, reads = 0;
-    int k = 0, d = 0, top = 0;
-    bool active = false;
-    if (valid && n >= 2) {
-        // The root is popped first, with an empty stack (d = 0).
-        const float4 R0 = __ldg(a.root), R1 = __ldg(a.root + 1);
-        active = apply_room(L, visit_child<COUNT, PHI>(L, W, a, R0, R1.x, n, s, true), 0, a.max_stack);
-    }
-    for (;;) {
-        if (!active) {
-            if (top == 0) break;
-            const unsigned e = (unsigned)lstk[(--top) * LANE_THREADS + tid];
-            k = (int)(e & ((1u << LANE_KBITS) - 1u));
-            d = (int)(e >> LANE_KBITS);
-            active = true;
-        }
-        if ((unsigned)k >= (unsigned)(n - 1)) {  // never for a consistent tree
-            ++bad;
-            break;
-        }
-        const ulonglong2 A = __ldg(reinterpret_cast<const ulonglong2 *>(a.inode + 3 * k));
-        const ulonglong2 B = __ldg(reinterpret_cast<const ulonglong2 *>(a.inode + 3 * k + 1));
-        const float4 C = __ldg(a.inode + 3 * k + 2);
-        if (COUNT) ++reads;
-        bool wantL, wantR;
-        visit_pair<COUNT, PHI>(L, W, a, A, B, C, s, true, E2, TH2, wantL, wantR);
-        if (PHI) W.self |= k == W.kp;
-        if (d + 3 > a.max_stack) {  // the rule only bites near max_stack
-            wantR = apply_room(L, wantR, d + 1, a.max_stack);
-            wantL = apply_room(L, wantL, d, a.max_stack);
-        }
-        if (wantR) {
-            if (wantL) {
-                if (top < a.max_stack) {
-                    lstk[(top++) * LANE_THREADS + tid] =
-                        (int)((unsigned)(__float_as_int(C.z) - n) | ((unsigned)d << LANE_KBITS));
-                } else {
-                    ++overflow;
-                }
-            }
-            k = __float_as_int(C.w) - n;
-            d = d + 1;
-        } else if (wantL) {
-            k = __float_as_int(C.z) - n;
-        } else {
-            active = false;
-        }
-    }
-    // Counters: one atomic per warp and counter.
-    unsigned dsum = L.drops, osum = overflow, bsum = bad;
-    const int lane = tid & 31;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        dsum += __shfl_xor_sync(0xffffffffu, dsum, o);
-        osum += __shfl_xor_sync(0xffffffffu, osum, o);
-        bsum += __shfl_xor_sync(0xffffffffu, bsum, o);
-    }
-    if (COUNT) {
-        unsigned isum = L.n_int, tsum = L.n_test, rsum = reads, vsum = (valid && n >= 2) ? 1u : 0u;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            isum += __shfl_xor_sync(0xffffffffu, isum, o);
-            tsum += __shfl_xor_sync(0xffffffffu, tsum, o);
-            rsum += __shfl_xor_sync(0xffffffffu, rsum, o);
-            vsum += __shfl_xor_sync(0xffffffffu, vsum, o);
-        }
-        if (lane == 0) {
-            atomicAdd(a.diag + DIAG_NODE_READS, (unsigned long long)rsum);
-            atomicAdd(a.diag + DIAG_ROOT_READS, (unsigned long long)vsum);
-            atomicAdd(a.diag + DIAG_INTERACTIONS, (unsigned long long)isum);
-            atomicAdd(a.diag + DIAG_TESTS, (unsigned long long)tsum);
-        }
-    }
-    if (lane == 0) {
-        if (dsum) atomicAdd(a.diag + DIAG_STACK_DROPS, (unsigned long long)dsum);
-        if (osum) atomicAdd(a.diag + DIAG_STACK_OVERFLOW, (unsigned long long)osum);
-        if (bsum) atomicAdd(a.diag + DIAG_BAD_TREE, (unsigned long long)bsum);
-    }
-    if (!valid) return;
-    const uint32_t p = __ldg(a.order + s);
-    if (p >= (uint32_t)n) return;
-    float xl, xr, yl, yr, zl, zr;
-    unpack2(L.AX, xl, xr);
-    unpack2(L.AY, yl, yr);
-    unpack2(L.AZ, zl, zr);
-    float gx = a.G * (L.ax + (xl + xr)), gy = a.G * (L.ay + (yl + yr)), gz = a.G * (L.az + (zl + zr));
-    if (a.pot.on) ext_acc_add(a.pot, L.px, L.py, L.pz, gx, gy, gz);
-    if (PHI) phi[p] = lane_phi(W, a.eps2);
+// The acceleration G s of particle p, the analytic potential's added (and the
+// closing kick), written at its own index: the traversals' epilogue.
+template <bool KDK>
+__device__ __forceinline__ void trav_write(const TravArgs &a, uint32_t p, float px, float py, float pz, float sx,
+                                           float sy, float sz) {
+    float gx = a.G * sx, gy = a.G * sy, gz = a.G * sz;
+    if (a.pot.on) ext_acc_add(a.pot, px, py, pz, gx, gy, gz);
     if (KDK) {
         const float4 vh = a.vel[p];
         a.vel[p] = make_float4(kick(vh.x, gx, a.h), kick(vh.y, gy, a.h), kick(vh.z, gz, a.h), vh.w);
@@ -482,6 +48,487 @@ bh_traverse_lane_kernel(TravArgs a, float *__restrict__ phi, const int *__restri
     } else {
         a.acc[p] = make_float4(gx, gy, gz, 0.f);
     }
+}
+
+// ----------------------------------------------------------- particle walk
+// Per-particle walk: T key-consecutive targets share a warp.  The nodes that
+// some target opened form a list in the order of the reference's walk (a
+// node, then its right subtree, then its left one); a round
+//   expands  up to 32 unexpanded nodes of the list, the first ones, one per
+//            lane: loads their two-children records and applies the
+//            reference's own test size^2 < theta^2 (|d|^2 + eps^2)
+//            (core/solvers/barnes_hut.py:204-210) of both children to all T
+//            targets, two targets per .f32x2 instruction, broadcast from
+//            shared memory.  An expanded node keeps the masks of the targets
+//            that accepted its children; an opened child enters the list
+//            behind it;
+//   emits    the expanded nodes at the list's head, up to the first
+//            unexpanded one, into a buffer of records;
+//   sums     a full buffer: every lane adds the records, in order, to its
+//            target; children outside the target's mask add zero.
+// So every target sums exactly the node set of the reference's _traverse
+// (:180-217), its accepted left children and its accepted right children
+// each in the order of the reference's walk, whatever its group: results
+// depend neither on T, nor on the range of targets, nor on scheduling.
+//
+// Leaves carry size^2 = -1 in the record, so the one comparison accepts every
+// leaf.  A target's own leaf (:198) sits at distance 0 and adds a zero force.
+// depth is the depth of the reference's per-particle stack when the node is
+// popped; it depends only on the node's path (a right child is popped at
+// depth + 1, a left child at depth), so the max_stack rule (:212) holds per
+// node, and the skipped pushes of all its targets are counted.
+//
+// The list cannot overflow: a round expands no more nodes than half the free
+// elements above WALK_RESERVE (an expanded node stays until it is emitted and
+// adds at most two), and at least one, the first, which the next round emits;
+// single expansions are a depth-first walk, which needs at most one more
+// element per tree level (63 key bits + 31 index bits) and two in all.
+//
+// Bound by issue: 67% of the slots at n = 400,000, the FMA pipe at 55%, the
+// shared-memory pipe at 69%.  1M disk, theta 0.5: 2.35 ms, against 3.40 ms for
+// a walk that expanded one node per warp step (74 instructions for 32
+// targets' tests and terms of a record, 61% of the lanes in use for the
+// tests and 31% for the terms); 100,000: 218 against 442 us; 10,000, theta
+// 0.6: 48 against 129 us for one walk per lane.  A round's test costs 344
+// instructions for 32 records, a summed record 23.  Measured on the disk:
+//   - T by n (us, theta 0.5): 4,000: 41.1 (T = 4), 44.3 (8); 8,000: 52.0,
+//     54.0; 12,000: 60.8 (8), 69.6 (16); 25,000: 87.6, 87.2; 50,000: 123
+//     (16), 157 (32); 70,000: 172, 172; 150,000: 346, 330; 1M: 2.69 ms, 2.35.
+//     Small groups give a small system more warps and shorter rounds, large
+//     ones share records and rounds among more targets.
+//   - CAP 512 with 10 CTAs per SM: 2.53 ms at 1M before the last two items,
+//     608 with 8: 2.64, 448 with 11: 2.61 (a short list expands fewer nodes
+//     per round, 24 of 32 lanes at 512).
+//   - a node that no target accepted a child of leaves the list: 2.82 to
+//     2.64 ms with the sums below it.
+//   - the buffer's sums and the list's chase between the record loads and the
+//     tests, emitted records stored a round later: 2.51 and 2.38 ms; eight
+//     records unrolled in the sums: 2.35.
+//   - asynchronous copies of the emitted records: 2.34 ms, but 6% slower below
+//     100,000; not kept.
+//   - sums in round order instead of the reference's: 1.71 ms, but the last
+//     bits then depend on the group, and over several steps a changed last
+//     bit flips acceptance tests; not kept.
+// Targets per group by n: 4, 8, 16 below these, then 32.
+constexpr int64_t WALK_4_N = 8192, WALK_8_N = 20480, WALK_16_N = 65536;
+constexpr int WALK_WARPS = 2;
+constexpr int WALK_RESERVE = 100;
+constexpr int WALK_LIST = 32;  // buffered records per warp
+template <int T>
+struct WalkShape {
+    static constexpr int CAP = 512;  // list elements; the last one ends the list
+    static constexpr int CTAS = T == 32 ? 10 : 11;   // resident CTAs per SM
+};
+
+template <int T>
+struct WalkWarp {
+    static constexpr int CAP = WalkShape<T>::CAP;
+    float4 tx[T / 4], ty[T / 4], tz[T / 4];  // the targets
+    // Buffered records: T = 32 the record's own {x_L, x_R, y_L, y_R} and
+    // {z_L, z_R, m_L, m_R}, else the left and the right child {x, y, z, m}.
+    float4 ra[WALK_LIST], rb[WALK_LIST];
+    uint2 rm[T == 32 ? WALK_LIST : 1];          // masks (left, right)
+    unsigned rmask[T == 32 ? 1 : WALK_LIST];    // left | right << T
+    // The list: node, masks (unexpanded: targets that opened it; expanded:
+    // that accepted the left and right child), next element, and flags
+    // (unexpanded: depth; expanded: 0x80).
+    int ek[CAP];
+    unsigned ea[CAP];
+    unsigned eb[T == 32 ? CAP : 1];
+    unsigned short nx[CAP];
+    // Free elements from the front; unexpanded ones, in list order, at the back.
+    unsigned short sf[CAP];
+    unsigned char fl[CAP];
+};
+
+// Two targets against one node: shifts the outcomes (1: accepted) of the
+// second and the first into the mask.  size^2 < t is the sign of size^2 - t,
+// which rounding keeps (a NaN's is positive: not accepted).  The difference
+// is an FMA by -1 (NEG, not known to the compiler), because the compiler
+// contracts a packed product and difference into one rounding.
+__device__ __forceinline__ unsigned walk_test(unsigned mask, f2 x, f2 y, f2 z, f2 TX, f2 TY, f2 TZ, f2 S2, f2 E2,
+                                              f2 TH2, f2 NEG) {
+    const f2 dx = sub2(x, TX), dy = sub2(y, TY), dz = sub2(z, TZ);
+    f2 r2 = fma2(dx, dx, E2);
+    r2 = fma2(dy, dy, r2);
+    r2 = fma2(dz, dz, r2);
+    float d0, d1;
+    unpack2(fma2(mul2(TH2, r2), NEG, S2), d0, d1);
+    mask = __funnelshift_l(__float_as_uint(d1), mask, 1);
+    return __funnelshift_l(__float_as_uint(d0), mask, 1);
+}
+
+// A lane's sums.  T = 32: packed over the (left, right) children; else the
+// lane's own side in the low half.
+struct WalkSum {
+    f2 X, Y, Z, W;
+};
+
+// Adds the buffered records [0, cnt) to the lane's target at (px, py, pz).
+template <bool PHI, int T>
+__device__ __forceinline__ void walk_eval(const WalkWarp<T> &w, int cnt, int lane, float px, float py, float pz,
+                                          float eps2, WalkSum &s) {
+    if constexpr (T == 32) {
+        const f2 PX = pack2(px, px), PY = pack2(py, py), PZ = pack2(pz, pz), E2 = pack2(eps2, eps2);
+        const unsigned bit = 1u << lane;
+        const ulonglong2 *RA = reinterpret_cast<const ulonglong2 *>(w.ra),
+                         *RB = reinterpret_cast<const ulonglong2 *>(w.rb);
+#pragma unroll 8
+        for (int i = 0; i < cnt; ++i) {
+            const ulonglong2 A = RA[i], B = RB[i];
+            const uint2 k = w.rm[i];
+            const f2 dx = sub2(A.x, PX), dy = sub2(A.y, PY), dz = sub2(B.x, PZ);
+            f2 r2 = fma2(dx, dx, E2);
+            r2 = fma2(dy, dy, r2);
+            r2 = fma2(dz, dz, r2);
+            const f2 inv = rsqrt2(r2);
+            float c0, c1;
+            unpack2(mul2(mul2(B.y, inv), mul2(inv, inv)), c0, c1);
+            const f2 sc = pack2((k.x & bit) ? c0 : 0.f, (k.y & bit) ? c1 : 0.f);
+            s.X = fma2(sc, dx, s.X);
+            s.Y = fma2(sc, dy, s.Y);
+            s.Z = fma2(sc, dz, s.Z);
+            if (PHI) s.W = fma2(sc, r2, s.W);
+        }
+    } else {
+        const unsigned bit = 1u << (lane & (2 * T - 1));
+        const float4 *R = (lane & T) ? w.rb : w.ra;
+        float sx, sy, sz, sw, none;
+        unpack2(s.X, sx, none);
+        unpack2(s.Y, sy, none);
+        unpack2(s.Z, sz, none);
+        unpack2(s.W, sw, none);
+#pragma unroll 8
+        for (int i = 0; i < cnt; ++i) {
+            const float4 q = R[i];
+            const unsigned k = w.rmask[i];
+            const float dx = __fsub_rn(q.x, px), dy = __fsub_rn(q.y, py), dz = __fsub_rn(q.z, pz);
+            const float r2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmaf_rn(dx, dx, eps2)));
+            const float inv = rsqrt_approx(r2);
+            const float c = __fmul_rn(__fmul_rn(q.w, inv), __fmul_rn(inv, inv));
+            const float sc = (k & bit) ? c : 0.f;
+            sx = __fmaf_rn(sc, dx, sx);
+            sy = __fmaf_rn(sc, dy, sy);
+            sz = __fmaf_rn(sc, dz, sz);
+            if (PHI) sw = __fmaf_rn(sc, r2, sw);
+        }
+        s.X = pack2(sx, 0.f);
+        s.Y = pack2(sy, 0.f);
+        s.Z = pack2(sz, 0.f);
+        s.W = pack2(sw, 0.f);
+    }
+}
+
+// left + right sum of a lane's target.
+template <int T>
+__device__ __forceinline__ float walk_total(f2 v) {
+    float lo, hi;
+    unpack2(v, lo, hi);
+    if (T < 32) hi = __shfl_xor_sync(0xffffffffu, lo, T);
+    return lo + hi;
+}
+
+template <bool KDK, bool COUNT, bool PHI, int T>
+__global__ void __launch_bounds__(WALK_WARPS * 32, WalkShape<T>::CTAS)
+bh_walk_kernel(TravArgs a, float *__restrict__ phi, int s0, int s1) {
+    constexpr int CAP = WalkShape<T>::CAP, END = CAP - 1;
+    extern __shared__ __align__(16) unsigned char walk_smem[];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    WalkWarp<T> &w = reinterpret_cast<WalkWarp<T> *>(walk_smem)[wid];
+    const int n = a.n;
+    const int g0 = s0 + (blockIdx.x * WALK_WARPS + wid) * T;  // the group's first target
+    if (g0 >= s1) return;  // whole warp out of range
+    const int gn = min(T, s1 - g0);
+    // The lane's target: g0 + t (T < 32: its left side in lanes t, its right
+    // side in lanes t + T).
+    const int t = lane & (T - 1);
+    float px = 0.f, py = 0.f, pz = 0.f, pm = 0.f;
+    if (t < gn) {
+        const float4 p = __ldg(a.leaf + g0 + t);
+        px = p.x; py = p.y; pz = p.z; pm = p.w;
+    }
+    if (lane < T) {
+        reinterpret_cast<float *>(w.tx)[lane] = px;
+        reinterpret_cast<float *>(w.ty)[lane] = py;
+        reinterpret_cast<float *>(w.tz)[lane] = pz;
+    }
+    const f2 E2 = pack2(a.eps2, a.eps2), TH2 = pack2(a.theta2, a.theta2);
+    const float neg = __int_as_float((int)0xBF800000 | (n >> 30));  // -1 (n < 2^30)
+    const f2 NEG = pack2(neg, neg);
+    const unsigned lt = (1u << lane) - 1u;
+    WalkSum sum;
+    sum.X = sum.Y = sum.Z = sum.W = 0ull;
+    unsigned drops = 0, bad = 0, reads = 0, n_int = 0, n_test = 0, self = 0;
+    float ax = 0.f, ay = 0.f, az = 0.f, aw = 0.f;  // the root's term
+    int ns = 0;     // unexpanded elements, the first at sf[CAP - ns]
+    int nfree = 0;  // free elements in sf[0 .. nfree)
+    int fresh = 0;  // elements never used: fresh .. END - 1
+    int head = END, live = 0, cnt = 0;
+    if (n >= 2) {
+        // The root is popped first, with an empty stack (depth 0).
+        const float4 R0 = __ldg(a.root), R1 = __ldg(a.root + 1);
+        const float dx = R0.x - px, dy = R0.y - py, dz = R0.z - pz;
+        const float r2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmaf_rn(dx, dx, a.eps2)));
+        const bool acc = R1.x < a.theta2 * r2;
+        if (acc) {
+            const float inv = rsqrt_approx(r2);
+            const float sc = R0.w * inv * inv * inv;
+            ax = __fmul_rn(sc, dx);
+            ay = __fmul_rn(sc, dy);
+            az = __fmul_rn(sc, dz);
+            aw = R0.w * inv;
+        }
+        const bool mine = lane < gn;
+        unsigned om = __ballot_sync(0xffffffffu, mine && !acc);
+        if (COUNT && lane == 0) {
+            n_int += gn - __popc(om);
+            n_test += gn;
+        }
+        if (a.max_stack < 2) {
+            drops += lane == 0 ? __popc(om) : 0;
+            om = 0;
+        }
+        if (lane == 0) {
+            w.nx[END] = END;
+            w.fl[END] = 0;
+            w.ek[0] = 0;
+            w.ea[0] = om;
+            w.fl[0] = 0;
+            w.nx[0] = END;
+            w.sf[END] = 0;
+        }
+        if (om) {
+            ns = live = fresh = 1;
+            head = 0;
+        }
+    }
+    __syncwarp();
+    // Emits the expanded elements among the first 32 of the list, of which lane
+    // i holds the i-th (h: the one after them), and frees their elements; lane
+    // i < cnt then has the i-th one's record in U, V and masks in uL, uR.
+    float4 U = make_float4(0.f, 0.f, 0.f, 0.f), V = U;
+    unsigned uL = 0, uR = 0;
+    auto emit = [&](int mine, int h, int got) {
+        const unsigned stop = __ballot_sync(0xffffffffu, !(w.fl[mine] & 0x80));
+        cnt = stop ? __ffs(stop) - 1 : 32;
+        head = cnt < got ? __shfl_sync(0xffffffffu, mine, cnt) : h;
+        if (lane < cnt) {
+            const float4 *rc = a.inode + 3 * (int64_t)w.ek[mine];
+            U = __ldg(rc);
+            V = __ldg(rc + 1);
+            uL = w.ea[mine];
+            if constexpr (T == 32) uR = w.eb[mine];
+            w.sf[nfree + lane] = (unsigned short)mine;
+        }
+        nfree += cnt;
+        live -= cnt;
+    };
+    auto buffer = [&]() {
+        if (lane < cnt) {
+            if constexpr (T == 32) {
+                w.ra[lane] = U;
+                w.rb[lane] = V;
+                w.rm[lane] = make_uint2(uL, uR);
+            } else {
+                w.ra[lane] = make_float4(U.x, U.z, V.x, V.z);
+                w.rb[lane] = make_float4(U.y, U.w, V.y, V.w);
+                w.rmask[lane] = uL;
+            }
+        }
+        __syncwarp();
+    };
+    // The list's first elements, the i-th in lane i's `mine`, as far as the
+    // expanded ones reach (in eights); h: the one after them.
+    auto chase = [&](int &mine, int &h) {
+        mine = END;
+        h = head;
+        int got = 0;
+        do {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                if (lane == got + i) mine = h;
+                h = w.nx[h];
+            }
+            got += 8;
+        } while (got < 32 && (w.fl[h] & 0x80));
+        return got;
+    };
+    // A consistent tree expands each internal node at most once per group,
+    // so more than n - 1 rounds mean a corrupted tree: stop.
+    for (int round = 0; ns > 0; ++round) {
+        const int take = min(ns, max(1, min(32, (CAP - WALK_RESERVE - live) >> 1)));
+        const bool act = lane < take;
+        const int e = act ? w.sf[CAP - ns + lane] : END;
+        int k = 0, depth = 0;
+        unsigned m = 0;
+        if (act) {
+            k = w.ek[e];
+            m = w.ea[e];
+            depth = w.fl[e];
+        }
+        ns -= take;
+        if (round >= n || (unsigned)k >= (unsigned)(n - 1)) {  // never for a consistent tree
+            bad += __popc(m);
+            k = 0;
+            m = 0;
+        }
+        // Idle lanes read record 0 with an empty mask.
+        const float4 *rec = a.inode + 3 * (int64_t)k;
+        const float4 A = __ldg(rec), B = __ldg(rec + 1), C = __ldg(rec + 2);
+        if (COUNT) reads += __popc(__ballot_sync(0xffffffffu, m != 0));
+        // While the records arrive: the list's head as the last round left it
+        // (a chain of shared-memory loads), and the buffer's sums.
+        int mine, h;
+        const int got = chase(mine, h);
+        buffer();
+        walk_eval<PHI>(w, cnt, lane, px, py, pz, a.eps2, sum);
+        unsigned aL = 0, aR = 0;
+        {
+            const f2 XL = pack2(A.x, A.x), YL = pack2(A.z, A.z), ZL = pack2(B.x, B.x), SL = pack2(C.x, C.x);
+            const f2 XR = pack2(A.y, A.y), YR = pack2(A.w, A.w), ZR = pack2(B.y, B.y), SR = pack2(C.y, C.y);
+            const ulonglong2 *TX = reinterpret_cast<const ulonglong2 *>(w.tx),
+                             *TY = reinterpret_cast<const ulonglong2 *>(w.ty),
+                             *TZ = reinterpret_cast<const ulonglong2 *>(w.tz);
+#pragma unroll
+            for (int j = T / 4 - 1; j >= 0; --j) {  // target 4 j + 3 first: its bit is shifted furthest
+                const ulonglong2 X = TX[j], Y = TY[j], Z = TZ[j];
+                aL = walk_test(aL, XL, YL, ZL, X.y, Y.y, Z.y, SL, E2, TH2, NEG);
+                aR = walk_test(aR, XR, YR, ZR, X.y, Y.y, Z.y, SR, E2, TH2, NEG);
+                aL = walk_test(aL, XL, YL, ZL, X.x, Y.x, Z.x, SL, E2, TH2, NEG);
+                aR = walk_test(aR, XR, YR, ZR, X.x, Y.x, Z.x, SR, E2, TH2, NEG);
+            }
+        }
+        emit(mine, h, got);
+        __syncwarp();
+        const int idL = __float_as_int(C.z), idR = __float_as_int(C.w);
+        unsigned oL = m & ~aL, oR = m & ~aR;
+        aL &= m;
+        aR &= m;
+        if (COUNT) {
+            n_int += __popc(aL) + __popc(aR);
+            n_test += (C.x >= 0.f ? __popc(m) : 0) + (C.y >= 0.f ? __popc(m) : 0);
+        }
+        if (idL < n) {
+            if (PHI || COUNT) {  // a target's own leaf
+                const unsigned o = (unsigned)(idL - g0) < (unsigned)T ? aL & (1u << (idL - g0)) : 0u;
+                self |= o;
+                if (COUNT && o) n_int -= 1u;
+            }
+            bad += __popc(oL);  // a leaf that fails the test has a non-finite distance
+            oL = 0;
+        }
+        if (idR < n) {
+            if (PHI || COUNT) {
+                const unsigned o = (unsigned)(idR - g0) < (unsigned)T ? aR & (1u << (idR - g0)) : 0u;
+                self |= o;
+                if (COUNT && o) n_int -= 1u;
+            }
+            bad += __popc(oR);
+            oR = 0;
+        }
+        if (depth + 3 > a.max_stack) {  // the rule only bites near max_stack
+            drops += __popc(oR);
+            oR = 0;
+            if (depth + 2 > a.max_stack) {
+                drops += __popc(oL);
+                oL = 0;
+            }
+        }
+        // The opened children in list order: right, left of lane 0, then of
+        // lane 1, ...  A node that no target accepted a child of leaves the
+        // list: its first opened child takes its element.  The others' are
+        // freed ones first, then fresh ones.
+        const unsigned cL = __ballot_sync(0xffffffffu, oL != 0), cR = __ballot_sync(0xffffffffu, oR != 0);
+        const bool swap = (aL | aR) == 0 && (oL | oR) != 0;
+        const unsigned cS = __ballot_sync(0xffffffffu, swap);
+        const int np = __popc(cL) + __popc(cR), na = np - __popc(cS);
+        if (fresh + max(0, na - nfree) > END) {  // never for a consistent tree
+            bad += lane == 0 ? 1u : 0u;
+            break;
+        }
+        const int rank = __popc(cL & lt) + __popc(cR & lt);
+        const int q = rank - __popc(cS & lt);  // the lane's first new element
+        const int n0 = q < nfree ? w.sf[nfree - 1 - q] : fresh + q - nfree;
+        const int n1 = q + 1 < nfree ? w.sf[nfree - 2 - q] : fresh + q + 1 - nfree;
+        __syncwarp();  // the popped and the free elements are read
+        ns += np;
+        live += na;
+        fresh += max(0, na - nfree);
+        nfree = max(0, nfree - na);
+        if (act) {
+            const int c1 = swap ? e : n0, c2 = swap ? n0 : n1;  // the first and the second opened child
+            int link = w.nx[e];
+            if (oL) {
+                const int el = oR ? c2 : c1;
+                w.ek[el] = idL - n;
+                w.ea[el] = oL;
+                w.fl[el] = (unsigned char)depth;
+                w.nx[el] = (unsigned short)link;
+                w.sf[CAP - ns + rank + (oR ? 1 : 0)] = (unsigned short)el;
+                link = el;
+            }
+            if (oR) {
+                w.ek[c1] = idR - n;
+                w.ea[c1] = oR;
+                w.fl[c1] = (unsigned char)(depth + 1);
+                w.nx[c1] = (unsigned short)link;
+                w.sf[CAP - ns + rank] = (unsigned short)c1;
+                link = c1;
+            }
+            if (!swap) {
+                w.nx[e] = (unsigned short)link;
+                w.fl[e] = 0x80;
+                if constexpr (T == 32) {
+                    w.ea[e] = aL;
+                    w.eb[e] = aR;
+                } else {
+                    w.ea[e] = aL | aR << T;
+                }
+            }
+        }
+        __syncwarp();
+    }
+    if (n >= 2) {  // the elements left are all expanded
+        do {
+            int mine, h;
+            const int got = chase(mine, h);
+            buffer();
+            walk_eval<PHI>(w, cnt, lane, px, py, pz, a.eps2, sum);
+            emit(mine, h, got);
+            __syncwarp();
+        } while (cnt > 0);
+    }
+    // Counters: one atomic per warp and counter.
+    const unsigned dsum = __reduce_add_sync(0xffffffffu, drops), bsum = __reduce_add_sync(0xffffffffu, bad);
+    if (lane == 0) {
+        if (dsum) atomicAdd(a.diag + DIAG_STACK_DROPS, (unsigned long long)dsum);
+        if (bsum) atomicAdd(a.diag + DIAG_BAD_TREE, (unsigned long long)bsum);
+    }
+    if (COUNT) {
+        const unsigned isum = __reduce_add_sync(0xffffffffu, n_int), tsum = __reduce_add_sync(0xffffffffu, n_test);
+        if (lane == 0) {
+            atomicAdd(a.diag + DIAG_NODE_READS, (unsigned long long)reads);
+            atomicAdd(a.diag + DIAG_ROOT_READS, 1ull);
+            atomicAdd(a.diag + DIAG_INTERACTIONS, (unsigned long long)isum);
+            atomicAdd(a.diag + DIAG_TESTS, (unsigned long long)tsum);
+        }
+    }
+    const float tx = walk_total<T>(sum.X), ty = walk_total<T>(sum.Y), tz = walk_total<T>(sum.Z);
+    float pw = 0.f;
+    if (PHI) {
+        // The records' terms include the target's own leaf: remove it.
+        pw = aw + walk_total<T>(sum.W);
+        if ((__reduce_or_sync(0xffffffffu, self) >> t) & 1u) {
+            const float inv = rsqrt_approx(a.eps2);
+            pw = __fmaf_rn(-((pm * inv) * (inv * inv)), a.eps2, pw);
+        }
+    }
+    if (lane >= gn) return;
+    const int s = g0 + lane;
+    const uint32_t p = __ldg(a.order + s);
+    if (p >= (uint32_t)n) return;
+    if (PHI) phi[p] = pw;
+    trav_write<KDK>(a, p, px, py, pz, ax + tx, ay + ty, az + tz);
 }
 
 // ------------------------------------------------------------- group walk
@@ -681,8 +728,6 @@ __device__ __forceinline__ void gw_group(GwWarp &w, const TravArgs &a, float *__
     unpack2(AX, xl, xr);
     unpack2(AY, yl, yr);
     unpack2(AZ, zl, zr);
-    float gx = a.G * (xl + xr), gy = a.G * (yl + yr), gz = a.G * (zl + zr);
-    if (a.pot.on) ext_acc_add(a.pot, px, py, pz, gx, gy, gz);
     if (PHI) {
         float wl, wr;
         unpack2(PW, wl, wr);
@@ -690,17 +735,7 @@ __device__ __forceinline__ void gw_group(GwWarp &w, const TravArgs &a, float *__
         if ((selfbits >> lane) & 1u) pw -= pm * rsqrt_approx(a.eps2);  // the term the list added
         phi[p] = pw;
     }
-    if (KDK) {
-        const float4 vh = a.vel[p];
-        a.vel[p] = make_float4(kick(vh.x, gx, a.h), kick(vh.y, gy, a.h), kick(vh.z, gz, a.h), vh.w);
-        a.acc[p] = make_float4(gx, gy, gz, 0.f);
-    } else if (a.accumulate) {
-        float4 o = a.acc[p];
-        o.x += gx; o.y += gy; o.z += gz;
-        a.acc[p] = o;
-    } else {
-        a.acc[p] = make_float4(gx, gy, gz, 0.f);
-    }
+    trav_write<KDK>(a, p, px, py, pz, xl + xr, yl + yr, zl + zr);
 }
 
 // Warp w walks the groups whose first leaf lies in [32 w, 32 w + 32) (gsize
