@@ -51,6 +51,57 @@ __device__ __forceinline__ long long np_trunc_i64(double t) {
     return __double2ll_rz(t);
 }
 
+__device__ __forceinline__ GridPart empty_part() {
+    GridPart p;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        p.mn[a] = INFINITY;
+        p.mx[a] = -INFINITY;
+    }
+    p.hmax = -INFINITY;
+    p.count = p.nonfinite = 0;
+    return p;
+}
+
+__device__ __forceinline__ GridPart merge_part(const GridPart &x, const GridPart &y) {
+    GridPart p;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        p.mn[a] = fminf(x.mn[a], y.mn[a]);
+        p.mx[a] = fmaxf(x.mx[a], y.mx[a]);
+    }
+    p.hmax = fmaxf(x.hmax, y.hmax);
+    p.count = x.count + y.count;
+    p.nonfinite = x.nonfinite + y.nonfinite;
+    return p;
+}
+
+// Merge of a CTA's threads' partials, complete in thread 0; w: one per warp.
+__device__ __forceinline__ GridPart cta_merge(GridPart p, GridPart *w) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        GridPart q;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            q.mn[a] = __shfl_xor_sync(0xffffffffu, p.mn[a], o);
+            q.mx[a] = __shfl_xor_sync(0xffffffffu, p.mx[a], o);
+        }
+        q.hmax = __shfl_xor_sync(0xffffffffu, p.hmax, o);
+        q.count = __shfl_xor_sync(0xffffffffu, p.count, o);
+        q.nonfinite = __shfl_xor_sync(0xffffffffu, p.nonfinite, o);
+        p = merge_part(p, q);
+    }
+    if ((threadIdx.x & 31) == 0) w[threadIdx.x >> 5] = p;
+    __syncthreads();
+    if (threadIdx.x == 0)
+        for (int k = 1; k < GRID_THREADS / 32; ++k) p = merge_part(p, w[k]);
+    return p;
+}
+
+// Bound by the latency of its tail, the merge and the FP64 divisions of the
+// geometry.  The last CTA's threads share the merge of the block partials: at
+// n = 1,000,000 11.6 us, against 66.9 us with 608 partials read one after the
+// other by one thread.
 __global__ void __launch_bounds__(GRID_THREADS)
 grid_reduce_kernel(const float4 *__restrict__ xm, const float *__restrict__ hsml, const int *__restrict__ is_star,
                    int64_t n, double min_radius, long long max_cells, GridPart *part, unsigned *ticket,
@@ -69,67 +120,46 @@ grid_reduce_kernel(const float4 *__restrict__ xm, const float *__restrict__ hsml
         hm = fmaxf(hm, hv);
         ++cnt;
     }
-    __shared__ float sm[7][GRID_THREADS / 32];
-    __shared__ unsigned long long sc[2][GRID_THREADS / 32];
+    __shared__ GridPart wpart[GRID_THREADS / 32];
     __shared__ bool last;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        mn0 = fminf(mn0, __shfl_xor_sync(0xffffffffu, mn0, o));
-        mn1 = fminf(mn1, __shfl_xor_sync(0xffffffffu, mn1, o));
-        mn2 = fminf(mn2, __shfl_xor_sync(0xffffffffu, mn2, o));
-        mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, o));
-        mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, o));
-        mx2 = fmaxf(mx2, __shfl_xor_sync(0xffffffffu, mx2, o));
-        hm = fmaxf(hm, __shfl_xor_sync(0xffffffffu, hm, o));
-        cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-        bad += __shfl_xor_sync(0xffffffffu, bad, o);
-    }
-    if (lane == 0) {
-        sm[0][wid] = mn0; sm[1][wid] = mn1; sm[2][wid] = mn2;
-        sm[3][wid] = mx0; sm[4][wid] = mx1; sm[5][wid] = mx2; sm[6][wid] = hm;
-        sc[0][wid] = cnt; sc[1][wid] = bad;
-    }
-    __syncthreads();
+    GridPart bp;
+    bp.mn[0] = mn0; bp.mn[1] = mn1; bp.mn[2] = mn2;
+    bp.mx[0] = mx0; bp.mx[1] = mx1; bp.mx[2] = mx2;
+    bp.hmax = hm;
+    bp.count = cnt;
+    bp.nonfinite = bad;
+    bp = cta_merge(bp, wpart);
     if (threadIdx.x == 0) {
-        GridPart bp;
-        for (int a = 0; a < 3; ++a) {
-            bp.mn[a] = INFINITY;
-            bp.mx[a] = -INFINITY;
-        }
-        bp.hmax = -INFINITY;
-        bp.count = bp.nonfinite = 0;
-        for (int w = 0; w < GRID_THREADS / 32; ++w) {
-            for (int a = 0; a < 3; ++a) {
-                bp.mn[a] = fminf(bp.mn[a], sm[a][w]);
-                bp.mx[a] = fmaxf(bp.mx[a], sm[3 + a][w]);
-            }
-            bp.hmax = fmaxf(bp.hmax, sm[6][w]);
-            bp.count += sc[0][w];
-            bp.nonfinite += sc[1][w];
-        }
         part[blockIdx.x] = bp;
         __threadfence();
         const unsigned t = atomicAdd(ticket, 1u);
         last = (t == gridDim.x - 1);
     }
     __syncthreads();
-    if (!last || threadIdx.x != 0) return;
-    // Last CTA: merge the block partials in block order and derive the grid.
+    if (!last) return;
+    // Last CTA: merge the block partials, one or a few per thread, and derive
+    // the grid.
     __threadfence();
-    *ticket = 0;  // ready for the next rebuild (stream-ordered)
-    float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY}, hmax = -INFINITY;
-    unsigned long long count = 0, nonfinite = 0;
-    for (unsigned b = 0; b < gridDim.x; ++b) {
+    bp = empty_part();
+    for (unsigned b = threadIdx.x; b < gridDim.x; b += GRID_THREADS) {
         const GridPart *q = part + b;  // written by other CTAs: read past L1
+        GridPart o;
+#pragma unroll
         for (int a = 0; a < 3; ++a) {
-            mn[a] = fminf(mn[a], __ldcg(q->mn + a));
-            mx[a] = fmaxf(mx[a], __ldcg(q->mx + a));
+            o.mn[a] = __ldcg(q->mn + a);
+            o.mx[a] = __ldcg(q->mx + a);
         }
-        hmax = fmaxf(hmax, __ldcg(&q->hmax));
-        count += __ldcg(&q->count);
-        nonfinite += __ldcg(&q->nonfinite);
+        o.hmax = __ldcg(&q->hmax);
+        o.count = __ldcg(&q->count);
+        o.nonfinite = __ldcg(&q->nonfinite);
+        bp = merge_part(bp, o);
     }
+    __syncthreads();  // wpart is read
+    bp = cta_merge(bp, wpart);
+    if (threadIdx.x != 0) return;
+    *ticket = 0;  // ready for the next rebuild (stream-ordered)
+    const float *mn = bp.mn, *mx = bp.mx, hmax = bp.hmax;
+    const unsigned long long count = bp.count, nonfinite = bp.nonfinite;
     GridGeom g = *geom;  // a rebuild without gas keeps the previous geometry
     g.ngas = (long long)count;
     g.active = count > 0 ? 1 : 0;
@@ -211,24 +241,66 @@ __global__ void grid_gsort_kernel(const uint32_t *__restrict__ vals, int64_t n, 
     gsort[p] = p < geom->ngas ? (int)vals[p] : 0;
 }
 
-// cell_start[c] = lower bound of c in the sorted gas keys (c <= n_cells);
-// 0 above n_cells, as the reference re-zeroes its field each rebuild.
-__global__ void grid_start_kernel(const uint32_t *__restrict__ keys, const GridGeom *__restrict__ geom,
-                                  long long max_cells, int *cell_start) {
-    const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c > max_cells || !geom->active) return;
-    const long long nc = geom->n_cells, ng = geom->ngas;
-    int out = 0;
-    if (c <= nc) {
-        long long lo = 0, hi = ng;  // first index in [0, ngas) with key >= c
-        while (lo < hi) {
-            const long long mid = (lo + hi) >> 1;
-            if ((long long)__ldg(keys + mid) < c) lo = mid + 1;
-            else hi = mid;
-        }
-        out = (int)lo;
+// First index in [0, n) with key >= c, found by a warp: 32 probes per step.
+__device__ __forceinline__ long long warp_lower_bound(const uint32_t *__restrict__ keys, long long n, long long c) {
+    const int lane = threadIdx.x & 31;
+    long long lo = 0, hi = n;
+    while (lo < hi) {
+        const long long step = (hi - lo + 32) / 33, at = lo + (lane + 1) * step - 1;
+        const int below = __popc(__ballot_sync(0xffffffffu, at < hi && (long long)__ldg(keys + at) < c));
+        hi = below < 32 ? min(hi, lo + (below + 1) * step - 1) : hi;
+        lo += below * step;
     }
-    cell_start[c] = out;
+    return lo;
+}
+
+// cell_start[c] = lower bound of c in the sorted gas keys (c <= n_cells);
+// 0 above n_cells, as the reference re-zeroes its field each rebuild.  A CTA
+// takes START_CELLS consecutive cells: two warps search for the range of
+// their keys, then every thread searches that range for its cells, all at
+// once.  Most CTAs hold few keys or none, and their cells need few steps;
+// the searches are chains of reads, so the chain is what counts.
+// At n = 1,000,000 (4,000,000 cells): 8.3 us, against 17.7 us with one search
+// over all keys (20 dependent reads) per cell, and 34.7 us with the range's
+// keys counted per cell in shared memory (dense cells put most keys in a few
+// CTAs).
+constexpr int START_CELLS = 1024;
+
+__global__ void __launch_bounds__(GRID_THREADS)
+grid_start_kernel(const uint32_t *__restrict__ keys, const GridGeom *__restrict__ geom, long long max_cells,
+                  int *__restrict__ cell_start) {
+    constexpr int PER = START_CELLS / GRID_THREADS;  // cells per thread
+    if (!geom->active) return;
+    __shared__ int range[2];
+    const int tid = threadIdx.x;
+    const long long c0 = (long long)blockIdx.x * START_CELLS;
+    const long long nc = geom->n_cells, ng = geom->ngas;
+    int at[PER];
+#pragma unroll
+    for (int q = 0; q < PER; ++q) at[q] = 0;
+    if (c0 <= nc) {
+        if (tid < 64) {
+            const int k = tid >> 5;
+            const long long r = warp_lower_bound(keys, ng, c0 + k * START_CELLS);
+            if ((tid & 31) == 0) range[k] = (int)r;
+        }
+        __syncthreads();
+        int len = range[1] - range[0];
+#pragma unroll
+        for (int q = 0; q < PER; ++q) at[q] = range[0];
+        while (len > 0) {
+            const int half = (len + 1) >> 1;
+#pragma unroll
+            for (int q = 0; q < PER; ++q)
+                if ((long long)__ldg(keys + at[q] + half - 1) < c0 + q * GRID_THREADS + tid) at[q] += half;
+            len -= half;
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < PER; ++q) {
+        const long long c = c0 + q * GRID_THREADS + tid;
+        if (c <= max_cells) cell_start[c] = c <= nc ? at[q] : 0;
+    }
 }
 
 }  // namespace gb
@@ -324,7 +396,7 @@ extern "C" int gb_grid_rebuild(gb_grid_t *h, const float *xm, const float *hsml,
                                                    h->vals[0]);
         const int cur = radix_sort_pairs<uint32_t>(h->keys, h->vals, n, h->passes, h->sort_scratch, h->diag, s);
         grid_gsort_kernel<<<g, GRID_THREADS, 0, s>>>(h->vals[cur], n, h->geom, gsort);
-        const unsigned gc = (unsigned)((h->max_cells + 1 + GRID_THREADS - 1) / GRID_THREADS);
+        const unsigned gc = (unsigned)((h->max_cells + START_CELLS) / START_CELLS);
         grid_start_kernel<<<gc, GRID_THREADS, 0, s>>>(h->keys[cur], h->geom, h->max_cells, cell_start);
         GB_CUDA_TRY(cudaGetLastError());
         h->launches += 4 + 1 + h->passes;
