@@ -36,11 +36,13 @@ namespace gb {
 struct BHParams {
     double lo[3];
     double scale;
+    float lof[3], sh, sl;  // the same for cell_fp32
 };
 
 
 
 constexpr int BBOX_THREADS = 256;
+constexpr int KEY_THREADS = 256;
 constexpr int BU_THREADS = 64;   // bottom-up CTA (a CTA retires with its longest ancestor chain)
 constexpr int MAX_DEPTH = 128;
 
@@ -48,7 +50,8 @@ constexpr int MAX_DEPTH = 128;
 template <bool KDK>
 __global__ void __launch_bounds__(BBOX_THREADS)
 bh_bbox_kernel(float4 *xm, float4 *vel, const float4 *acc, int64_t n, float h, float dt, float4 *part,
-               unsigned *ticket, BHParams *prm, int bits, unsigned long long *diag) {
+               unsigned *ticket, BHParams *prm, int bits, uint32_t *zero, int64_t nzero, unsigned long long *diag) {
+    rs_zero(zero, nzero);  // the sort's scratch
     float mn0 = INFINITY, mn1 = INFINITY, mn2 = INFINITY;
     float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY;
     unsigned long long bad = 0;
@@ -141,7 +144,12 @@ bh_bbox_kernel(float4 *xm, float4 *vel, const float4 *acc, int64_t n, float h, f
     prm->lo[0] = lo0;
     prm->lo[1] = lo1;
     prm->lo[2] = lo2;
-    prm->scale = __ddiv_rn(qmax, __dmul_rn(span, 1.0000001));
+    const double scale = __ddiv_rn(qmax, __dmul_rn(span, 1.0000001));
+    prm->scale = scale;
+    prm->lof[0] = a.x;
+    prm->lof[1] = a.y;
+    prm->lof[2] = a.z;
+    split_fp32(scale, prm->sh, prm->sl);
     *ticket = 0u;
 }
 
@@ -157,26 +165,38 @@ __device__ __forceinline__ uint64_t interleave3(uint32_t x, uint32_t y, uint32_t
     return r;
 }
 
-__device__ __forceinline__ uint32_t quantise(float x, double lo, double scale, double qmax) {
+// The FP64 quantisation, where FP32 cannot decide.
+__device__ __noinline__ uint32_t quantise_fp64(float x, double lo, double scale, double qmax) {
     double t = __dmul_rn(__dsub_rn((double)x, lo), scale);
     t = t > qmax ? qmax : t;
     t = t >= 0.0 ? t : 0.0;  // also maps NaN to 0 (counted in the bbox pass)
     return __double2uint_rz(t);
 }
 
+// Keys and, beside them, the digit counts of the sort (4 CTAs per SM share the
+// particles, so that a CTA counts many keys before it adds them up).  1M
+// particles, 30-bit keys: 11.2 us, against 35.1 us for FP64 keys alone and
+// 16.4 us for a kernel that counted their digits.
 template <typename KeyT, int BITS>
-__global__ void bh_morton_kernel(const float4 *__restrict__ xm, int64_t n, const BHParams *__restrict__ prm,
-                                 KeyT *__restrict__ keys, uint32_t *__restrict__ vals) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double qmax = (double)((1ull << BITS) - 1ull);
-    const double sc = prm->scale;
-    const float4 x = xm[i];
-    const uint32_t qx = quantise(x.x, prm->lo[0], sc, qmax);
-    const uint32_t qy = quantise(x.y, prm->lo[1], sc, qmax);
-    const uint32_t qz = quantise(x.z, prm->lo[2], sc, qmax);
-    keys[i] = (KeyT)interleave3<BITS>(qx, qy, qz);
-    vals[i] = (uint32_t)i;
+__global__ void __launch_bounds__(KEY_THREADS)
+bh_morton_kernel(const float4 *__restrict__ xm, int64_t n, const BHParams *__restrict__ prm,
+                 KeyT *__restrict__ keys, uint32_t *__restrict__ counts) {
+    constexpr int PASSES = (3 * BITS + 7) / 8;
+    constexpr uint32_t QMAX = (1u << BITS) - 1u;
+    __shared__ RsCount<PASSES> cnt;
+    cnt.clear();
+    const float lo0 = prm->lof[0], lo1 = prm->lof[1], lo2 = prm->lof[2], sh = prm->sh, sl = prm->sl;
+    for (int64_t i = (int64_t)blockIdx.x * KEY_THREADS + threadIdx.x; i < n; i += (int64_t)gridDim.x * KEY_THREADS) {
+        const float4 x = xm[i];
+        uint32_t qx, qy, qz;
+        if (!cell_fp32(x.x, lo0, sh, sl, qx)) qx = quantise_fp64(x.x, prm->lo[0], prm->scale, (double)QMAX);
+        if (!cell_fp32(x.y, lo1, sh, sl, qy)) qy = quantise_fp64(x.y, prm->lo[1], prm->scale, (double)QMAX);
+        if (!cell_fp32(x.z, lo2, sh, sl, qz)) qz = quantise_fp64(x.z, prm->lo[2], prm->scale, (double)QMAX);
+        const KeyT key = (KeyT)interleave3<BITS>(min(qx, QMAX), min(qy, QMAX), min(qz, QMAX));
+        keys[i] = key;
+        cnt.add(key, PASSES);
+    }
+    cnt.flush(counts, PASSES);
 }
 
 // ----------------------------------------------------------------- gather
@@ -596,19 +616,22 @@ static int build_impl(gb_bh_t *h, float4 *xm, float4 *vel, const float4 *acc, in
     const int nblk = std::max(1, std::min(h->bbox_blocks, (int)((n + BBOX_THREADS - 1) / BBOX_THREADS)));
     if (kdk)
         bh_bbox_kernel<true><<<nblk, BBOX_THREADS, 0, s>>>(xm, vel, acc, n, 0.5f * dt, dt, h->bbox_part, h->ticket,
-                                                           h->prm, BITS, h->diag);
+                                                           h->prm, BITS, h->sort_scratch, radix_zero_words(n),
+                                                           h->diag);
     else
         bh_bbox_kernel<false><<<nblk, BBOX_THREADS, 0, s>>>(xm, nullptr, nullptr, n, 0.f, 0.f, h->bbox_part,
-                                                            h->ticket, h->prm, BITS, h->diag);
+                                                            h->ticket, h->prm, BITS, h->sort_scratch,
+                                                            radix_zero_words(n), h->diag);
     const unsigned g256 = (unsigned)((n + 255) / 256);
     KeyT *k0 = (KeyT *)h->keys[0], *k1 = (KeyT *)h->keys[1];
     uint32_t *v0 = h->vals[0], *v1 = h->vals[1];
-    bh_morton_kernel<KeyT, BITS><<<g256, 256, 0, s>>>(xm, n, h->prm, k0, v0);
+    const unsigned gk = std::min((unsigned)(h->sms * 4), (unsigned)((n + KEY_THREADS - 1) / KEY_THREADS));
+    bh_morton_kernel<KeyT, BITS><<<gk, KEY_THREADS, 0, s>>>(xm, n, h->prm, k0, h->sort_scratch);
     mark(h, slot, 1, s);
     const int passes = (3 * BITS + 7) / 8;
     KeyT *kk[2] = {k0, k1};
     uint32_t *vv[2] = {v0, v1};
-    h->cur = radix_sort_pairs<KeyT>(kk, vv, n, passes, h->sort_scratch, h->diag, s);
+    h->cur = radix_sort_counted<KeyT>(kk, vv, n, passes, h->sort_scratch, h->diag, s);
     k0 = kk[h->cur];
     v0 = vv[h->cur];
     mark(h, slot, 2, s);
@@ -627,7 +650,7 @@ static int build_impl(gb_bh_t *h, float4 *xm, float4 *vel, const float4 *acc, in
     }
     GB_CUDA_TRY(cudaGetLastError());
     mark(h, slot, 4, s);
-    h->launches += 5 + 1 + passes - (n >= 2 ? 0 : 1);
+    h->launches += 5 + passes - (n >= 2 ? 0 : 1);
     h->n = n;
     return GB_OK;
 }

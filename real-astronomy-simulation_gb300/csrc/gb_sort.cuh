@@ -1,8 +1,8 @@
 // Stable LSD radix sort of (key, 32-bit value) pairs, 8-bit digits, shared by
 // the tree build (Morton keys) and the neighbour grid (cell keys).
 //
-// One histogram kernel counts the digits of every pass in a single read of
-// the keys.  Each pass is then one kernel: a CTA takes the next tile of 2048
+// The kernel that makes the keys counts the digits of every pass as it writes
+// them (RsCount).  Each pass is then one kernel: a CTA takes the next tile of 2048
 // keys from a counter, ranks them stably in index order (digit ballots within
 // a warp, warp offsets within the tile), stages the tile in shared memory in
 // digit order (so that global writes run in contiguous digit runs),
@@ -118,34 +118,43 @@ __device__ __forceinline__ uint32_t warp_digit_peers(uint32_t dig, bool ok, int 
     return ok ? m : (1u << lane);
 }
 
-// Digit counts of all passes: counts[p * 256 + digit] += keys with that
-// digit p (bits 8p .. 8p + 7).  Warp-aggregated shared-memory counts, then
-// one global add per non-zero bin and CTA.
-template <typename KeyT>
-__global__ void __launch_bounds__(RS_THREADS)
-rs_histogram_kernel(const KeyT *__restrict__ keys, int64_t n, int passes, uint32_t *__restrict__ counts) {
-    __shared__ uint32_t h[RS_MAX_PASSES * RS_BINS];
-    for (int i = threadIdx.x; i < passes * RS_BINS; i += RS_THREADS) h[i] = 0;
-    __syncthreads();
-    const int lane = threadIdx.x & 31;
-    const uint32_t lt_mask = (1u << lane) - 1u;
-    const int64_t stride = (int64_t)gridDim.x * RS_THREADS;
-    // Every lane of a warp runs the same number of rounds (the ballots need them all).
-    for (int64_t i0 = (int64_t)blockIdx.x * RS_THREADS + (threadIdx.x & ~31); i0 < n; i0 += stride) {
-        const int64_t i = i0 + lane;
-        const bool ok = i < n;
-        const KeyT k = ok ? keys[i] : (KeyT)0;
-        for (int p = 0; p < passes; ++p) {
-            const uint32_t dig = (uint32_t)(k >> (8 * p)) & 0xFFu;
-            const uint32_t peers = warp_digit_peers(dig, ok, lane);
-            if (ok && (peers & lt_mask) == 0) atomicAdd(&h[p * RS_BINS + dig], (uint32_t)__popc(peers));
+// Digit counts of all passes, taken by the kernel that makes the keys (it
+// starts with all scratch words of radix_zero_words zero): counts[p * 256 +
+// digit] += keys with that digit p (bits 8p .. 8p + 7).  Counted in shared
+// memory, in COPIES copies by lane (equal digits of a warp's keys meet fewer
+// conflicts), then one global add per non-zero bin and CTA.  A separate kernel
+// that read the keys again took 16.4 us at n = 1,000,000 (8 ballots per digit).
+template <int PASSES>
+struct RsCount {
+    static constexpr int COPIES = PASSES <= 4 ? 4 : 2;
+    uint32_t h[COPIES][PASSES * RS_BINS];
+
+    __device__ __forceinline__ void clear() {
+        for (int i = threadIdx.x; i < COPIES * PASSES * RS_BINS; i += blockDim.x) (&h[0][0])[i] = 0u;
+        __syncthreads();
+    }
+    template <typename KeyT>
+    __device__ __forceinline__ void add(KeyT k, int passes) {
+        uint32_t *c = h[threadIdx.x & (COPIES - 1)];
+#pragma unroll
+        for (int p = 0; p < PASSES; ++p)
+            if (p < passes) atomicAdd(c + p * RS_BINS + ((uint32_t)(k >> (8 * p)) & 0xFFu), 1u);
+    }
+    __device__ __forceinline__ void flush(uint32_t *counts, int passes) {
+        __syncthreads();
+        for (int i = threadIdx.x; i < passes * RS_BINS; i += blockDim.x) {
+            uint32_t n = 0;
+#pragma unroll
+            for (int q = 0; q < COPIES; ++q) n += h[q][i];
+            if (n) atomicAdd(counts + i, n);
         }
     }
-    __syncthreads();
-    for (int i = threadIdx.x; i < passes * RS_BINS; i += RS_THREADS) {
-        const uint32_t c = h[i];
-        if (c) atomicAdd(counts + i, c);
-    }
+};
+
+// Zeroes the first nz scratch words (a kernel that runs before the keys').
+__device__ __forceinline__ void rs_zero(uint32_t *scratch, int64_t nz) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nz; i += (int64_t)gridDim.x * blockDim.x)
+        scratch[i] = 0u;
 }
 
 // Exclusive scan of 256 values held one per thread of a 256-thread CTA.
@@ -178,8 +187,9 @@ __device__ __forceinline__ uint32_t cta256_exclusive_scan(uint32_t v, uint32_t *
 // digits; the destination is the digit's global start (scan of this pass's
 // counts) + the digit's count in earlier tiles (look-back) + the rank within
 // the tile.  status holds this pass's tile words (zeroed); status_next, when
-// given, is zeroed here for the next pass.
-template <typename KeyT>
+// given, is zeroed here for the next pass.  IOTA (the first pass): the values
+// are the keys' indices and are not read.
+template <typename KeyT, bool IOTA>
 __global__ void __launch_bounds__(RS_THREADS, 4)
 rs_onesweep_kernel(const KeyT *__restrict__ kin, const uint32_t *__restrict__ vin, KeyT *__restrict__ kout,
                    uint32_t *__restrict__ vout, int64_t n, int shift, const uint32_t *__restrict__ counts,
@@ -215,7 +225,7 @@ rs_onesweep_kernel(const KeyT *__restrict__ kin, const uint32_t *__restrict__ vi
         const int64_t i = wbase + r * 32 + lane;
         const bool ok = i < n;
         key[r] = ok ? kin[i] : (KeyT)0;
-        val[r] = ok ? vin[i] : 0u;
+        val[r] = IOTA ? (uint32_t)i : (ok ? vin[i] : 0u);
         const uint32_t dig = (uint32_t)(key[r] >> shift) & 0xFFu;
         const uint32_t peers = warp_digit_peers(dig, ok, lane);
         const uint32_t before = ok ? whist[wid][dig] : 0u;
@@ -269,28 +279,34 @@ rs_onesweep_kernel(const KeyT *__restrict__ kin, const uint32_t *__restrict__ vi
     }
 }
 
-// Sorts (k[0], v[0]) by the low 8 * passes bits of the keys (n < 2^30,
-// passes <= 8), ping-ponging with (k[1], v[1]); returns the index of the
-// pair holding the result.  scratch holds radix_scratch_size(n) words.
-// Launches: one memset, the histogram kernel and one kernel per pass.
+// Scratch words that are zero when the kernel that makes the keys starts:
+// the digit counts, the tile counters and the first pass's status array.
+inline int64_t radix_zero_words(int64_t n) {
+    return (int64_t)RS_MAX_PASSES * RS_BINS + RS_COUNTERS + radix_tiles(n) * RS_BINS;
+}
+
+// Sorts k[0], with the indices 0 .. n - 1 as values, by the low 8 * passes
+// bits of the keys (n < 2^30, 1 <= passes <= 8), ping-ponging with k[1] and
+// v; returns the index of the pair holding the result.  scratch holds
+// radix_scratch_size(n) words, zeroed (radix_zero_words) and with the digit
+// counts added (RsCount).  Launches: one kernel per pass.
 template <typename KeyT>
-static int radix_sort_pairs(KeyT *k[2], uint32_t *v[2], int64_t n, int passes, uint32_t *scratch,
-                            unsigned long long *diag, cudaStream_t s) {
-    if (n <= 0 || passes <= 0) return 0;
+static int radix_sort_counted(KeyT *k[2], uint32_t *v[2], int64_t n, int passes, uint32_t *scratch,
+                              unsigned long long *diag, cudaStream_t s) {
     const int nb = (int)radix_tiles(n);
     uint32_t *counts = scratch;
     uint32_t *counters = counts + RS_MAX_PASSES * RS_BINS;
     uint32_t *status[2] = {counters + RS_COUNTERS, counters + RS_COUNTERS + (int64_t)nb * RS_BINS};
-    cudaMemsetAsync(scratch, 0, sizeof(uint32_t) * ((int64_t)RS_MAX_PASSES * RS_BINS + RS_COUNTERS + (int64_t)nb * RS_BINS),
-                    s);
-    const int hb = (int)std::min<int64_t>((n + RS_THREADS - 1) / RS_THREADS, 4 * (int64_t)num_sms());
-    rs_histogram_kernel<KeyT><<<hb, RS_THREADS, 0, s>>>(k[0], n, passes, counts);
     int cur = 0;
     for (int p = 0; p < passes; ++p) {
         uint32_t *next = p + 1 < passes ? status[(p + 1) & 1] : nullptr;
-        rs_onesweep_kernel<KeyT><<<nb, RS_THREADS, 0, s>>>(k[cur], v[cur], k[cur ^ 1], v[cur ^ 1], n, 8 * p,
-                                                           counts + p * RS_BINS, counters + p, status[p & 1], next,
-                                                           nb, diag);
+        if (p == 0)
+            rs_onesweep_kernel<KeyT, true><<<nb, RS_THREADS, 0, s>>>(k[0], v[0], k[1], v[1], n, 0, counts, counters,
+                                                                     status[0], next, nb, diag);
+        else
+            rs_onesweep_kernel<KeyT, false><<<nb, RS_THREADS, 0, s>>>(k[cur], v[cur], k[cur ^ 1], v[cur ^ 1], n, 8 * p,
+                                                                      counts + p * RS_BINS, counters + p, status[p & 1],
+                                                                      next, nb, diag);
         cur ^= 1;
     }
     return cur;
