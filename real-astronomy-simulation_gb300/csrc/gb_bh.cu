@@ -10,15 +10,13 @@
 //               interleave x,y,z into bits 3b, 3b+1, 3b+2
 //   2 sort      stable LSD radix sort (8-bit digits) of (key, index): the
 //               permutation of np.argsort(kind="stable") (:247)
-//   3 gather    particles into key order (leaf records)
-//   4 karras    binary radix tree, identical to _build_radix (:84-121)
-//   5 bottom-up node mass, first moment and AABB (FP32); a node is
-//               summarised by the second of its two children to finish
-//               (integer arrival ticket with acquire-release ordering, L2
-//               reads): no floating-point atomics, and the result is
-//               independent of scheduling (:124-177 use FP64 atomics on
-//               every ancestor instead)
-//   6 traverse  per-particle walk: 4 to 32 key-consecutive targets share a
+//   3 tree      particles into key order (leaf records), the binary radix
+//               tree, identical to _build_radix (:84-121), and node mass,
+//               first moment and AABB (FP32) in one pass upwards, in shared
+//               memory within chunks of leaves; no floating-point atomics,
+//               and the result is independent of scheduling (:124-177 use
+//               FP64 atomics on every ancestor instead)
+//   4 traverse  per-particle walk: 4 to 32 key-consecutive targets share a
 //               warp and its list of opened nodes; every target applies the reference's own acceptance
 //               test size^2 < theta^2 (r^2 + eps^2) (:204-210), so each
 //               particle accepts exactly the node set of _traverse
@@ -43,15 +41,13 @@ struct BHParams {
 
 constexpr int BBOX_THREADS = 256;
 constexpr int KEY_THREADS = 256;
-constexpr int BU_THREADS = 64;   // bottom-up CTA (a CTA retires with its longest ancestor chain)
-constexpr int MAX_DEPTH = 128;
 
 // ------------------------------------------------------------------ bbox
 template <bool KDK>
 __global__ void __launch_bounds__(BBOX_THREADS)
 bh_bbox_kernel(float4 *xm, float4 *vel, const float4 *acc, int64_t n, float h, float dt, float4 *part,
-               unsigned *ticket, BHParams *prm, int bits, uint32_t *zero, int64_t nzero, unsigned long long *diag) {
-    rs_zero(zero, nzero);  // the sort's scratch
+               unsigned *ticket, BHParams *prm, int bits, ZeroWords zero, unsigned long long *diag) {
+    zero_words(zero);
     float mn0 = INFINITY, mn1 = INFINITY, mn2 = INFINITY;
     float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY;
     unsigned long long bad = 0;
@@ -199,21 +195,7 @@ bh_morton_kernel(const float4 *__restrict__ xm, int64_t n, const BHParams *__res
     cnt.flush(counts, PASSES);
 }
 
-// ----------------------------------------------------------------- gather
-__global__ void bh_gather_kernel(const float4 *__restrict__ xm, const uint32_t *__restrict__ order, int64_t n,
-                                 float4 *__restrict__ leaf, unsigned long long *diag) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const uint32_t o = order[i];
-    if (o < n) {
-        leaf[i] = __ldg(xm + o);
-    } else {
-        leaf[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        atomicAdd(diag + DIAG_BAD_TREE, 1ull);
-    }
-}
-
-// ----------------------------------------------------------------- karras
+// ------------------------------------------------------------------ tree
 // Common-prefix length of keys i and j over bits 62..0; equal keys continue
 // with the index bits 30..0 (63 + prefix); -1 outside [0, n) (:71-81).
 __device__ __forceinline__ int clz63(uint64_t x) { return __clzll(x) - 1; }
@@ -227,54 +209,6 @@ __device__ __forceinline__ int kdelta(const KeyT *__restrict__ k, int n, int i, 
     return clz63(x);
 }
 
-// Leaves per group of the group walk (traversal shape 3).
-constexpr int GW_GROUP = 32;
-
-// gsize (when not NULL, zeroed before the launch): the group walk's groups,
-// the maximal subtrees with at most GW_GROUP leaves; gsize[first leaf] =
-// its leaf count.  They partition the leaves into key-order ranges, each
-// inside one node's box (32 key-consecutive leaves can straddle a jump of
-// the Morton curve and span most of the system).
-template <typename KeyT>
-__global__ void bh_karras_kernel(const KeyT *__restrict__ k, int n, int2 *__restrict__ child,
-                                 int *__restrict__ parent, int *__restrict__ gsize) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i == 0) parent[n] = -1;  // the root (internal node 0 = id n)
-    if (i >= n - 1) return;
-    const int d = kdelta(k, n, i, i + 1) > kdelta(k, n, i, i - 1) ? 1 : -1;
-    const int d_min = kdelta(k, n, i, i - d);
-    int l_max = 2;
-    while (kdelta(k, n, i, i + l_max * d) > d_min) l_max *= 2;
-    int l = 0;
-    for (int t = l_max / 2; t >= 1; t /= 2)
-        if (kdelta(k, n, i, i + (l + t) * d) > d_min) l += t;
-    const int j = i + l * d;
-    const int d_node = kdelta(k, n, i, j);
-    int s = 0;
-    int t2 = (l + 1) / 2;
-    while (t2 >= 1) {
-        if (kdelta(k, n, i, i + (s + t2) * d) > d_node) s += t2;
-        t2 = t2 > 1 ? (t2 + 1) / 2 : 0;
-    }
-    const int gamma = i + s * d + min(d, 0);
-    const int lo = min(i, j), hi = max(i, j);
-    const int lc = (lo == gamma) ? gamma : gamma + n;
-    const int rc = (hi == gamma + 1) ? gamma + 1 : gamma + 1 + n;
-    child[i] = make_int2(lc, rc);
-    parent[lc] = i + n;
-    parent[rc] = i + n;
-    if (gsize) {
-        const int cnt = hi - lo + 1, cl = gamma - lo + 1, cr = hi - gamma;
-        if (cnt > GW_GROUP) {
-            if (cl <= GW_GROUP) gsize[lo] = cl;
-            if (cr <= GW_GROUP) gsize[gamma + 1] = cr;
-        } else if (i == 0) {
-            gsize[0] = cnt;  // the whole system is one group
-        }
-    }
-}
-
-// -------------------------------------------------------------- bottom-up
 // Node summary in FP32: mass, first moment about the node's AABB minimum
 // corner, and the AABB.  Moments about the corner keep the centre of mass
 // accurate to rounding of the node size (a cluster of coincident particles
@@ -285,24 +219,24 @@ struct NodeSum {
     float lx, ly, lz, hx, hy, hz;
 };
 
-__device__ __forceinline__ NodeSum child_sum(int c, int n, const float4 *__restrict__ leaf,
-                                             const float4 *__restrict__ sums, const float4 *__restrict__ bmin,
-                                             const float4 *__restrict__ bmax) {
+__device__ __forceinline__ NodeSum leaf_sum(float4 p) {
     NodeSum s;
-    if (c < n) {
-        const float4 p = __ldg(leaf + c);
-        s.m = p.w;
-        s.sx = s.sy = s.sz = 0.f;
-        s.lx = s.hx = p.x;
-        s.ly = s.hy = p.y;
-        s.lz = s.hz = p.z;
-    } else {
-        const int k = c - n;
-        const float4 q = __ldcg(sums + k), a = __ldcg(bmin + k), b = __ldcg(bmax + k);
-        s.m = q.x; s.sx = q.y; s.sy = q.z; s.sz = q.w;
-        s.lx = a.x; s.ly = a.y; s.lz = a.z;
-        s.hx = b.x; s.hy = b.y; s.hz = b.z;
-    }
+    s.m = p.w;
+    s.sx = s.sy = s.sz = 0.f;
+    s.lx = s.hx = p.x;
+    s.ly = s.hy = p.y;
+    s.lz = s.hz = p.z;
+    return s;
+}
+
+__device__ __forceinline__ NodeSum merge_sums(const NodeSum &a, const NodeSum &b) {
+    NodeSum s;
+    s.lx = fminf(a.lx, b.lx); s.ly = fminf(a.ly, b.ly); s.lz = fminf(a.lz, b.lz);
+    s.hx = fmaxf(a.hx, b.hx); s.hy = fmaxf(a.hy, b.hy); s.hz = fmaxf(a.hz, b.hz);
+    s.m = a.m + b.m;
+    s.sx = __fmaf_rn(b.m, b.lx - s.lx, __fmaf_rn(a.m, a.lx - s.lx, a.sx + b.sx));
+    s.sy = __fmaf_rn(b.m, b.ly - s.ly, __fmaf_rn(a.m, a.ly - s.ly, a.sy + b.sy));
+    s.sz = __fmaf_rn(b.m, b.lz - s.lz, __fmaf_rn(a.m, a.lz - s.lz, a.sz + b.sz));
     return s;
 }
 
@@ -319,75 +253,403 @@ __device__ __forceinline__ float size2_of(const NodeSum &s) {
     return e * e;
 }
 
-// Arrival ticket with acquire-release ordering at GPU scope: the first child
-// to finish publishes its summary; the second observes it.
-__device__ __forceinline__ unsigned arrive(unsigned *p) {
-    unsigned old;
-    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(old) : "l"(p) : "memory");
-    return old;
-}
+// The binary radix tree and its summaries in one kernel (the reference's
+// _build_radix and summary passes, core/solvers/barnes_hut.py:84-177).
+//
+// The internal node that splits its leaves between g and g + 1 joins the two
+// subtrees that end at g and start at g + 1, and a subtree over leaves [l, r]
+// is a left child, split at r, when its keys share more with leaf r + 1 than
+// with leaf l - 1, else a right child, split at l - 1 (Apetrei, "Fast and
+// Simple Agglomerative LBVH Construction", 2014).  In the numbering of the
+// reference (Karras) a left child has index r, a right child index l and the
+// root 0.  So a node's place, parent and children follow from its leaf range
+// alone, and its summary from its children's: leaves, topology and summaries
+// need one pass upwards and no searches.
+//
+// A CTA joins its TREE_CHUNK consecutive leaves in shared memory: a subtree
+// that comes to the split of its parent first stays there, and the second
+// makes the parent.  While there are many parents to make they are queued and
+// spread over the CTA, round by round; the last 32 each take a lane of one
+// warp and go upwards on their own.  What is left are the maximal subtrees inside the chunk, at most one per tree
+// level and side (a dozen or two in practice).  The last CTA of TREE_GROUP
+// chunks to finish takes the subtrees of all of them as the leaves of the
+// same procedure, and so on up to the root.  No floating-point atomics, and
+// no CTA waits for another; the result does not depend on scheduling (the
+// reference uses FP64 atomics on every ancestor).  The merge keeps its
+// operands' order, so results are those of a node-by-node pass, bit for bit.
+//
+// Bound by latency: that of the levels in shared memory and of the hand-over
+// between CTAs.  Disk, 63-bit keys to 100,000, 30-bit above (us): 10,000: 20;
+// 100,000: 34; 300,000: 44; 1M: 102, against 57, 72, 98 and 211 for a gather,
+// a search-based topology pass and a pass with one global arrival ticket per
+// node.  Measured at 10,000 / 1M (us): tickets at every node, topology from
+// ranges: 59 / 155; nodes of a chunk in queued rounds, records inside: 47 /
+// 168; records apart: 27 / 129; one thread per leaf upwards instead of
+// rounds: 24 / 122; rounds down to 32 nodes: 20 / 105; 4 CTAs per SM (64
+// registers): 20 / 102.  128 threads: 27 / 110; 512: 18 / 152.
+constexpr int TREE_THREADS = 256;
+constexpr int TREE_CHUNK = 512;   // leaves or subtrees joined at a time
+constexpr int TREE_GROUP = 32;    // units of a level that the next one joins (one per lane)
+constexpr int TREE_PEND = 192;    // subtrees left of a unit (63 key bits + 31 index bits on each side)
+// Leaves per group of the group walk (traversal shape 3).
+constexpr int GW_GROUP = 32;
 
-// True for the second child to arrive.  A sibling that already arrived is
-// seen by an acquire load, which synchronises with its release and needs no
-// fence of the caller's own stores: those are released by the atomic at the
-// first node where the caller arrives first, the only place it stops.
-__device__ __forceinline__ bool second_arrival(unsigned *p) {
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v != 0u || arrive(p) != 0u;
-}
+// A finished subtree over leaves [l, r] and the common prefixes beyond its ends.
+struct alignas(16) TreeItem {
+    NodeSum s;
+    int l, r, dl, dr;
+};
 
-// Summarises every internal node k once both children are done and writes
-// the traversal record of its two children as (left, right) pairs:
+struct TreeArgs {
+    const float4 *xm;
+    const uint32_t *order;
+    int n;
+    float4 *leaf;
+    int2 *child;
+    int *parent;
+    // Subtrees left of every unit (level after level, TREE_PEND each), their
+    // number, and the finished units of every group (zero at launch).
+    TreeItem *items;
+    int *count;
+    unsigned *done;
+    float4 *sums, *bmin, *bmax, *inode, *root;
+    // The group walk's groups, when it is asked for (NULL or zero at launch):
+    // the maximal subtrees with at most GW_GROUP leaves; gsize[first leaf] =
+    // its leaf count.  They partition the leaves into key-order ranges, each
+    // inside one node's box (32 key-consecutive leaves can straddle a jump of
+    // the Morton curve and span most of the system).
+    int *gsize;
+    unsigned long long *diag;
+};
+
+// Writes the node of leaves [l, r] split at p, with index k; s: its summary, a
+// and b: its children's.  The traversal record of k holds its two children as
+// (left, right) pairs:
 //   inode[3k] = {x_L, x_R, y_L, y_R}, inode[3k+1] = {z_L, z_R, m_L, m_R},
 //   inode[3k+2] = {size2_L, size2_R, id_L, id_R} (ids as bits; size2 = -1
-//   marks a leaf child), so the traversal loads both children pre-packed for
-//   .f32x2 arithmetic.
-// Bounded for 20 resident CTAs per SM: 48 registers (a 20-byte spill)
-// against 56 registers and 18 CTAs without the bound (1M disk: 181 against
-// 184 us; 4M: 542 against 567 us).
-__global__ void __launch_bounds__(BU_THREADS, 20) bh_bottomup_kernel(const float4 *__restrict__ leaf, const int2 *__restrict__ child,
-                                   const int *__restrict__ parent, int n, unsigned *__restrict__ arrivals,
-                                   float4 *__restrict__ sums, float4 *__restrict__ bmin, float4 *__restrict__ bmax,
-                                   float4 *__restrict__ inode, float4 *__restrict__ root, unsigned long long *diag) {
-    const int li = blockIdx.x * blockDim.x + threadIdx.x;
-    if (li >= n) return;
-    int node = __ldg(parent + li);
-    for (int depth = 0; node >= 0; ++depth) {
-        if (depth >= MAX_DEPTH || node < n || node >= 2 * n - 1) {
-            atomicAdd(diag + DIAG_BAD_TREE, 1ull);
-            return;
+//   marks a leaf child), pre-packed for .f32x2 arithmetic.
+__device__ __forceinline__ void tree_record(const TreeArgs &t, const NodeSum &s, const NodeSum &a, const NodeSum &b,
+                                            int l, int r, int p, int k) {
+    const int n = t.n;
+    const int lc = l == p ? p : p + n, rc = r == p + 1 ? r : p + 1 + n;
+    t.child[k] = make_int2(lc, rc);
+    t.parent[lc] = k + n;
+    t.parent[rc] = k + n;
+    t.sums[k] = make_float4(s.m, s.sx, s.sy, s.sz);
+    t.bmin[k] = make_float4(s.lx, s.ly, s.lz, 0.f);
+    t.bmax[k] = make_float4(s.hx, s.hy, s.hz, 0.f);
+    const float4 ca = trav_com(a), cb = trav_com(b);
+    t.inode[3 * (int64_t)k] = make_float4(ca.x, cb.x, ca.y, cb.y);
+    t.inode[3 * (int64_t)k + 1] = make_float4(ca.z, cb.z, ca.w, cb.w);
+    t.inode[3 * (int64_t)k + 2] = make_float4(l == p ? -1.f : size2_of(a), r == p + 1 ? -1.f : size2_of(b),
+                                              __int_as_float(lc), __int_as_float(rc));
+    const bool is_root = l == 0 && r == n - 1;
+    if (is_root) {
+        t.root[0] = trav_com(s);
+        t.root[1] = make_float4(size2_of(s), 0.f, 0.f, 0.f);
+        t.parent[n] = -1;
+    }
+    if (t.gsize) {
+        const int cnt = r - l + 1, cl = p - l + 1, cr = r - p;
+        if (cnt > GW_GROUP) {
+            if (cl <= GW_GROUP) t.gsize[l] = cl;
+            if (cr <= GW_GROUP) t.gsize[p + 1] = cr;
+        } else if (is_root) {
+            t.gsize[0] = cnt;  // the whole system is one group
         }
-        const int k = node - n;
-        if (!second_arrival(arrivals + k)) return;  // the sibling subtree is still running
-        const int2 c = __ldg(child + k);
-        if ((unsigned)c.x >= (unsigned)(2 * n - 1) || (unsigned)c.y >= (unsigned)(2 * n - 1)) {
-            atomicAdd(diag + DIAG_BAD_TREE, 1ull);
-            return;
-        }
-        const NodeSum a = child_sum(c.x, n, leaf, sums, bmin, bmax);
-        const NodeSum b = child_sum(c.y, n, leaf, sums, bmin, bmax);
+    }
+}
+
+struct TreeShared {
+    // Summaries: of the leaves or subtrees to join (the items), then of the
+    // nodes above them, each at the place of its first or last item (as the
+    // node is a right or a left child), whose own summary is then in use no
+    // more except in the records.
+    float sum[10][TREE_CHUNK];
+    float4 leaf[TREE_CHUNK];                  // the items, while they are leaves
+    int first[TREE_CHUNK], last[TREE_CHUNK];  // their leaf ranges
+    // Per split (j lies before item j; 0 and m are the outer ones): 1 + the
+    // first item of the left child that came, and 1 + the last item of the
+    // right one in the upper half.
+    unsigned came[TREE_CHUNK + 1];
+    signed char delta[TREE_CHUNK + 1];        // per split: common prefix of the leaves beside it
+    unsigned queue[2][TREE_CHUNK / 2];        // nodes to make: first item | last item << 10 | split << 20
+    int queued[3];
+    short end[TREE_CHUNK];
+    int scan[TREE_THREADS / 32];
+    int before[TREE_GROUP + 1];               // subtrees of the units before each one of a group
+    bool last_unit;
+
+    __device__ __forceinline__ NodeSum get(int i) const {
         NodeSum s;
-        s.lx = fminf(a.lx, b.lx); s.ly = fminf(a.ly, b.ly); s.lz = fminf(a.lz, b.lz);
-        s.hx = fmaxf(a.hx, b.hx); s.hy = fmaxf(a.hy, b.hy); s.hz = fmaxf(a.hz, b.hz);
-        s.m = a.m + b.m;
-        s.sx = __fmaf_rn(b.m, b.lx - s.lx, __fmaf_rn(a.m, a.lx - s.lx, a.sx + b.sx));
-        s.sy = __fmaf_rn(b.m, b.ly - s.ly, __fmaf_rn(a.m, a.ly - s.ly, a.sy + b.sy));
-        s.sz = __fmaf_rn(b.m, b.lz - s.lz, __fmaf_rn(a.m, a.lz - s.lz, a.sz + b.sz));
-        sums[k] = make_float4(s.m, s.sx, s.sy, s.sz);
-        bmin[k] = make_float4(s.lx, s.ly, s.lz, 0.f);
-        bmax[k] = make_float4(s.hx, s.hy, s.hz, 0.f);
-        const float4 ca = trav_com(a), cb = trav_com(b);
-        inode[3 * k] = make_float4(ca.x, cb.x, ca.y, cb.y);
-        inode[3 * k + 1] = make_float4(ca.z, cb.z, ca.w, cb.w);
-        inode[3 * k + 2] = make_float4(c.x < n ? -1.f : size2_of(a), c.y < n ? -1.f : size2_of(b),
-                                       __int_as_float(c.x), __int_as_float(c.y));
-        const int up = __ldg(parent + node);
-        if (up < 0) {
-            root[0] = trav_com(s);
-            root[1] = make_float4(size2_of(s), 0.f, 0.f, 0.f);
+        s.m = sum[0][i]; s.sx = sum[1][i]; s.sy = sum[2][i]; s.sz = sum[3][i];
+        s.lx = sum[4][i]; s.ly = sum[5][i]; s.lz = sum[6][i];
+        s.hx = sum[7][i]; s.hy = sum[8][i]; s.hz = sum[9][i];
+        return s;
+    }
+    __device__ __forceinline__ void put(int i, const NodeSum &s) {
+        sum[0][i] = s.m; sum[1][i] = s.sx; sum[2][i] = s.sy; sum[3][i] = s.sz;
+        sum[4][i] = s.lx; sum[5][i] = s.ly; sum[6][i] = s.lz;
+        sum[7][i] = s.hx; sum[8][i] = s.hy; sum[9][i] = s.hz;
+    }
+};
+
+// The subtree over the items [a, b] comes to the split of its parent (not the
+// root).  Returns whether it is the second there: then [a, b] is the parent's
+// range and j its split.
+__device__ __forceinline__ bool tree_come(TreeShared &w, bool left, int &a, int &b, int &j) {
+    j = left ? b + 1 : a;
+    __threadfence_block();  // its summary first
+    const unsigned old = atomicOr(&w.came[j], left ? (unsigned)(a + 1) : (unsigned)(b + 1) << 16);
+    const int sib = (int)(left ? old >> 16 : old & 0xFFFFu) - 1;
+    if (sib < 0) return false;  // the sibling is not there yet, or lies outside
+    __threadfence_block();
+    if (left) b = sib;
+    else a = sib;
+    return true;
+}
+
+// Makes the node over the items [a, b], split at j; false for the root.
+__device__ __forceinline__ bool tree_make(TreeShared &w, int a, int b, int j, bool &left) {
+    const int da = w.delta[a], db = w.delta[b + 1];
+    left = db > da;
+    w.put(left ? b : a, merge_sums(w.get(j - 1), w.get(j)));
+    return da >= 0 || db >= 0;
+}
+
+// Joins the m items in w (summaries, leaf ranges, deltas; m >= 1) as far as
+// they reach.  Complete after the barrier at its end.
+__device__ __forceinline__ void tree_join(TreeShared &w, int m) {
+    const int tid = threadIdx.x;
+    for (int i = tid; i <= m; i += TREE_THREADS) w.came[i] = 0u;
+    if (tid < 3) w.queued[tid] = 0;
+    __syncthreads();
+    auto push = [&](int a, int b, int j, int q, int c) {
+        w.queue[q][atomicAdd(&w.queued[c], 1)] = (unsigned)a | (unsigned)b << 10 | (unsigned)j << 20;
+    };
+    for (int i = tid; i < m; i += TREE_THREADS) {
+        int a = i, b = i, j;
+        const int da = w.delta[i], db = w.delta[i + 1];
+        if ((da >= 0 || db >= 0) && tree_come(w, db > da, a, b, j)) push(a, b, j, 0, 0);
+    }
+    __syncthreads();
+    int q = 0, c = 0;
+    for (;;) {
+        const int ready = w.queued[c], c1 = c == 2 ? 0 : c + 1;
+        if (ready <= 32) break;
+        if (tid == 0) w.queued[c1 == 2 ? 0 : c1 + 1] = 0;  // read one round ago, used by the next one
+        for (int i = tid; i < ready; i += TREE_THREADS) {
+            const unsigned e = w.queue[q][i];
+            int a = (int)(e & 1023u), b = (int)(e >> 10 & 1023u), j = (int)(e >> 20);
+            bool left;
+            if (tree_make(w, a, b, j, left) && tree_come(w, left, a, b, j)) push(a, b, j, q ^ 1, c1);
         }
-        node = up;
+        __syncthreads();
+        q ^= 1;
+        c = c1;
+    }
+    if (tid < w.queued[c]) {  // 32 at most: a lane each
+        const unsigned e = w.queue[q][tid];
+        int a = (int)(e & 1023u), b = (int)(e >> 10 & 1023u), j = (int)(e >> 20);
+        bool left;
+        while (tree_make(w, a, b, j, left) && tree_come(w, left, a, b, j)) {
+        }
+    }
+    __syncthreads();
+}
+
+// The records of the nodes that tree_join made; base(i): the summary of item
+// i.  Apart from the joining, because the divisions of the centres and the 13
+// stores of a node would lengthen every level.
+template <typename F>
+__device__ __forceinline__ void tree_records(const TreeShared &w, const TreeArgs &t, int m, F base) {
+    for (int j = threadIdx.x + 1; j < m; j += TREE_THREADS) {
+        const int a = (int)(w.came[j] & 0xFFFFu) - 1, b = (int)(w.came[j] >> 16) - 1;
+        if (a < 0 || b < 0) continue;
+        const int da = w.delta[a], db = w.delta[b + 1], l = w.first[a], r = w.last[b];
+        const bool left = db > da;
+        const NodeSum x = a == j - 1 ? base(a) : w.get(j - 1), y = b == j ? base(b) : w.get(j);
+        tree_record(t, w.get(left ? b : a), x, y, l, r, w.last[j - 1], da < 0 && db < 0 ? 0 : left ? r : l);
+    }
+}
+
+// Writes the subtrees that are left, in leaf order, to dst; returns how many.
+__device__ __forceinline__ int tree_left(TreeShared &w, TreeItem *dst, int m) {
+    constexpr int PER = TREE_CHUNK / TREE_THREADS;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    for (int i = tid; i < TREE_CHUNK; i += TREE_THREADS) w.end[i] = 0;  // 1 + the last item of the subtree from here
+    __syncthreads();
+    for (int j = tid; j <= m; j += TREE_THREADS) {
+        const int a = (int)(w.came[j] & 0xFFFFu) - 1, b = (int)(w.came[j] >> 16) - 1;
+        if (a >= 0 && b < 0) w.end[a] = (short)j;
+        else if (b >= 0 && a < 0) w.end[j] = (short)(b + 1);
+    }
+    __syncthreads();
+    int own = 0;
+#pragma unroll
+    for (int q = 0; q < PER; ++q) own += w.end[tid * PER + q] != 0;
+    int inc = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += v;
+    }
+    if (lane == 31) w.scan[wid] = inc;
+    __syncthreads();
+    int at = inc - own, total = 0;
+#pragma unroll
+    for (int k = 0; k < TREE_THREADS / 32; ++k) {
+        if (k < wid) at += w.scan[k];
+        total += w.scan[k];
+    }
+#pragma unroll
+    for (int q = 0; q < PER; ++q) {
+        const int a = tid * PER + q, b = w.end[a] - 1;
+        if (b < 0) continue;
+        TreeItem x;
+        x.dl = w.delta[a];
+        x.dr = w.delta[b + 1];
+        x.s = w.get(x.dr > x.dl ? b : a);
+        x.l = w.first[a];
+        x.r = w.last[b];
+        dst[at++] = x;
+    }
+    return total;
+}
+
+__device__ __forceinline__ void tree_take(TreeShared &w, const TreeItem &x, int i, bool last) {
+    w.put(i, x.s);
+    w.first[i] = x.l;
+    w.last[i] = x.r;
+    w.delta[i] = (signed char)x.dl;
+    if (last) w.delta[i + 1] = (signed char)x.dr;
+}
+
+__device__ __forceinline__ TreeItem load_item(const TreeItem *p) {  // written by other CTAs: read past L1
+    static_assert(sizeof(TreeItem) == 64, "four 16-byte loads");
+    union {
+        float4 v[4];
+        TreeItem x;
+    } u;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) u.v[k] = __ldcg(reinterpret_cast<const float4 *>(p) + k);
+    return u.x;
+}
+
+template <typename KeyT>
+__global__ void __launch_bounds__(TREE_THREADS, 4) bh_tree_kernel(const KeyT *__restrict__ keys, TreeArgs t) {
+    __shared__ TreeShared w;
+    const int tid = threadIdx.x, n = t.n;
+    int unit = blockIdx.x, units = gridDim.x, base = 0, groups = 0;  // units and groups of the levels below
+    int m = min(TREE_CHUNK, n - unit * TREE_CHUNK);
+    for (int i = tid; i <= m; i += TREE_THREADS) {
+        const int g = unit * TREE_CHUNK + i;
+        w.delta[i] = g >= 1 ? (signed char)kdelta(keys, n, g - 1, g) : (signed char)-1;
+        if (i == m) continue;
+        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (t.order) {
+            const uint32_t o = t.order[g];
+            if (o < (uint32_t)n) x = __ldg(t.xm + o);
+            else atomicAdd(t.diag + DIAG_BAD_TREE, 1ull);
+            t.leaf[g] = x;
+        } else {
+            x = t.leaf[g];
+        }
+        w.leaf[i] = x;
+        w.put(i, leaf_sum(x));
+        w.first[i] = w.last[i] = g;
+    }
+    if (n == 1) {  // the root is the leaf
+        if (tid == 0) t.parent[0] = t.parent[1] = -1;
+        return;
+    }
+    __syncthreads();
+    tree_join(w, m);
+    if (units == 1) {
+        tree_records(w, t, m, [&](int i) { return leaf_sum(w.leaf[i]); });
+        return;
+    }
+    TreeItem *items = nullptr;  // the items of levels above the leaves
+    bool apart = true;          // unit u's at items[u * TREE_PEND ..], not back to back
+    auto item = [&](int i) {
+        if (!apart) return items + i;
+        int u = 0;
+#pragma unroll
+        for (int o = TREE_GROUP / 2; o > 0; o >>= 1)
+            if (i >= w.before[u + o]) u += o;
+        return items + u * TREE_PEND + (i - w.before[u]);
+    };
+    auto above = [&](int i) { return load_item(item(i)).s; };
+    for (int level = 0; units > 1; ++level) {
+        const int left = tree_left(w, t.items + (int64_t)(base + unit) * TREE_PEND, m);
+        // The last unit of the group to finish goes on with all of its
+        // subtrees; the records are written while that is being found out.
+        static_assert(TREE_GROUP == 32, "one unit of a group per lane");
+        const int group = unit / TREE_GROUP, gn = min(TREE_GROUP, units - group * TREE_GROUP);
+        __syncthreads();
+        if (tid == 0) {
+            t.count[base + unit] = left;
+            __threadfence();
+            w.last_unit = atomicAdd(t.done + groups + group, 1u) == (unsigned)(gn - 1);
+        }
+        if (level == 0) tree_records(w, t, m, [&](int i) { return leaf_sum(w.leaf[i]); });
+        else tree_records(w, t, m, above);
+        __syncthreads();
+        if (!w.last_unit) return;
+        __threadfence();
+        if (tid < 32) {
+            int c = tid < gn ? __ldcg(t.count + base + group * TREE_GROUP + tid) : 0;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, c, o);
+                if (tid >= o) c += v;
+            }
+            w.before[tid + 1] = c;
+            if (tid == 0) w.before[0] = 0;
+        }
+        __syncthreads();
+        items = t.items + (int64_t)(base + group * TREE_GROUP) * TREE_PEND;
+        apart = true;
+        int total = w.before[TREE_GROUP];
+        // More than fit (trees far deeper than log2 n): join them piece by
+        // piece; a piece leaves fewer than half its items, which go back to
+        // the front of the same storage.
+        while (total > TREE_CHUNK) {
+            int out = 0;
+            for (int i0 = 0; i0 < total; i0 += TREE_CHUNK) {
+                m = min(TREE_CHUNK, total - i0);
+                __syncthreads();
+                for (int i = tid; i < m; i += TREE_THREADS) tree_take(w, load_item(item(i0 + i)), i, i == m - 1);
+                __syncthreads();
+                tree_join(w, m);
+                tree_records(w, t, m, [&](int i) { return load_item(item(i0 + i)).s; });
+                __syncthreads();  // the items are read
+                out += tree_left(w, items + out, m);
+            }
+            __syncthreads();
+            __threadfence();
+            apart = false;
+            total = out;
+        }
+        __syncthreads();
+        m = total;
+        for (int i = tid; i < m; i += TREE_THREADS) tree_take(w, load_item(item(i)), i, i == m - 1);
+        __syncthreads();
+        tree_join(w, m);
+        base += units;
+        groups += (units + TREE_GROUP - 1) / TREE_GROUP;
+        unit = group;
+        units = (units + TREE_GROUP - 1) / TREE_GROUP;
+    }
+    tree_records(w, t, m, above);
+}
+
+// Units and groups of all levels for n leaves.
+static void tree_units(int64_t n, int64_t *units, int64_t *groups) {
+    *units = *groups = 0;
+    for (int64_t u = (n + TREE_CHUNK - 1) / TREE_CHUNK; u > 1; u = (u + TREE_GROUP - 1) / TREE_GROUP) {
+        *units += u;
+        *groups += (u + TREE_GROUP - 1) / TREE_GROUP;
     }
 }
 
@@ -485,7 +747,9 @@ struct gb_bh {
     float4 *leaf;
     int2 *child;
     int *parent;
-    unsigned *arrivals;
+    TreeItem *tree_items;  // scratch of the build between chunks
+    int *tree_count;
+    unsigned *tree_done;
     float4 *sums;
     float4 *bmin, *bmax;
     float4 *inode;
@@ -538,7 +802,7 @@ static size_t key_size(int bits) { return bits <= 10 ? sizeof(uint32_t) : sizeof
 extern "C" int gb_bh_destroy(gb_bh_t *h) {
     if (!h) return GB_OK;
     void *ptrs[] = {h->keys[0], h->keys[1], h->vals[0], h->vals[1], h->sort_scratch, h->bbox_part, h->ticket,
-                    h->prm, h->leaf, h->child, h->parent, h->arrivals, h->sums, h->bmin, h->bmax,
+                    h->prm, h->leaf, h->child, h->parent, h->tree_items, h->tree_count, h->tree_done, h->sums, h->bmin, h->bmax,
                     h->inode, h->root, h->diag, h->epart, h->gsize};
     for (void *p : ptrs)
         if (p) cudaFree(p);
@@ -584,7 +848,11 @@ extern "C" int gb_bh_create(gb_bh_t **out, int64_t n_max, int key_bits) {
     A((void **)&h->leaf, sizeof(float4) * nn);
     A((void **)&h->child, sizeof(int2) * ni);
     A((void **)&h->parent, sizeof(int) * nodes);
-    A((void **)&h->arrivals, sizeof(unsigned) * ni);
+    int64_t units, groups;
+    tree_units(n_max, &units, &groups);
+    A((void **)&h->tree_items, sizeof(TreeItem) * TREE_PEND * std::max<int64_t>(units, 1));
+    A((void **)&h->tree_count, sizeof(int) * std::max<int64_t>(units, 1));
+    A((void **)&h->tree_done, sizeof(unsigned) * std::max<int64_t>(groups, 1));
     A((void **)&h->sums, sizeof(float4) * ni);
     A((void **)&h->bmin, sizeof(float4) * ni);
     A((void **)&h->bmax, sizeof(float4) * ni);
@@ -609,48 +877,66 @@ extern "C" int gb_bh_create(gb_bh_t **out, int64_t n_max, int key_bits) {
     return GB_OK;
 }
 
+// The tree over the handle's sorted keys; groups: also marks the group walk's
+// groups.  order: the particles of xm in key order; NULL: the leaves are there
+// already.  h->tree_done (and h->gsize) are zero.
+template <typename KeyT>
+static int build_tree(gb_bh_t *h, const float4 *xm, const uint32_t *order, int64_t n, bool groups, cudaStream_t s) {
+    TreeArgs t;
+    t.xm = xm;
+    t.order = order;
+    t.n = (int)n;
+    t.leaf = h->leaf;
+    t.child = h->child;
+    t.parent = h->parent;
+    t.items = h->tree_items;
+    t.count = h->tree_count;
+    t.done = h->tree_done;
+    t.sums = h->sums;
+    t.bmin = h->bmin;
+    t.bmax = h->bmax;
+    t.inode = h->inode;
+    t.root = h->root;
+    t.gsize = groups ? h->gsize : nullptr;
+    t.diag = h->diag;
+    bh_tree_kernel<KeyT><<<(unsigned)((n + TREE_CHUNK - 1) / TREE_CHUNK), TREE_THREADS, 0, s>>>(
+        (const KeyT *)h->keys[h->cur], t);
+    GB_CUDA_TRY(cudaGetLastError());
+    h->groups_n = groups ? n : -1;
+    h->launches += 1;
+    return GB_OK;
+}
+
 template <typename KeyT, int BITS>
 static int build_impl(gb_bh_t *h, float4 *xm, float4 *vel, const float4 *acc, int64_t n, float dt, bool kdk,
                       cudaStream_t s, int slot) {
     mark(h, slot, 0, s);
     const int nblk = std::max(1, std::min(h->bbox_blocks, (int)((n + BBOX_THREADS - 1) / BBOX_THREADS)));
+    // The sort's scratch, the tree's finished units and the group walk's marks.
+    const bool groups = h->tpl == 3;
+    int64_t units, ngroups;
+    tree_units(n, &units, &ngroups);
+    const ZeroWords zero = {{h->sort_scratch, h->tree_done, (uint32_t *)h->gsize},
+                            {radix_zero_words(n), ngroups, groups ? n : 0}};
     if (kdk)
         bh_bbox_kernel<true><<<nblk, BBOX_THREADS, 0, s>>>(xm, vel, acc, n, 0.5f * dt, dt, h->bbox_part, h->ticket,
-                                                           h->prm, BITS, h->sort_scratch, radix_zero_words(n),
-                                                           h->diag);
+                                                           h->prm, BITS, zero, h->diag);
     else
         bh_bbox_kernel<false><<<nblk, BBOX_THREADS, 0, s>>>(xm, nullptr, nullptr, n, 0.f, 0.f, h->bbox_part,
-                                                            h->ticket, h->prm, BITS, h->sort_scratch,
-                                                            radix_zero_words(n), h->diag);
-    const unsigned g256 = (unsigned)((n + 255) / 256);
-    KeyT *k0 = (KeyT *)h->keys[0], *k1 = (KeyT *)h->keys[1];
-    uint32_t *v0 = h->vals[0], *v1 = h->vals[1];
+                                                            h->ticket, h->prm, BITS, zero, h->diag);
+    KeyT *kk[2] = {(KeyT *)h->keys[0], (KeyT *)h->keys[1]};
     const unsigned gk = std::min((unsigned)(h->sms * 4), (unsigned)((n + KEY_THREADS - 1) / KEY_THREADS));
-    bh_morton_kernel<KeyT, BITS><<<gk, KEY_THREADS, 0, s>>>(xm, n, h->prm, k0, h->sort_scratch);
+    bh_morton_kernel<KeyT, BITS><<<gk, KEY_THREADS, 0, s>>>(xm, n, h->prm, kk[0], h->sort_scratch);
     mark(h, slot, 1, s);
     const int passes = (3 * BITS + 7) / 8;
-    KeyT *kk[2] = {k0, k1};
-    uint32_t *vv[2] = {v0, v1};
-    h->cur = radix_sort_counted<KeyT>(kk, vv, n, passes, h->sort_scratch, h->diag, s);
-    k0 = kk[h->cur];
-    v0 = vv[h->cur];
+    h->cur = radix_sort_counted<KeyT>(kk, h->vals, n, passes, h->sort_scratch, h->diag, s);
     mark(h, slot, 2, s);
-    bh_gather_kernel<<<g256, 256, 0, s>>>(xm, v0, n, h->leaf, h->diag);
-    const int ni = (int)std::max<int64_t>(n - 1, 1);
     // The group walk's groups are marked when the handle walks groups.
-    int *gsize = h->tpl == 3 ? h->gsize : nullptr;
-    if (gsize) GB_CUDA_TRY(cudaMemsetAsync(gsize, 0, sizeof(int) * n, s));
-    bh_karras_kernel<KeyT><<<(ni + 255) / 256, 256, 0, s>>>(k0, (int)n, h->child, h->parent, gsize);
-    h->groups_n = gsize ? n : -1;
+    GB_TRY(build_tree<KeyT>(h, xm, h->vals[h->cur], n, groups, s));
     mark(h, slot, 3, s);
-    if (n >= 2) {
-        GB_CUDA_TRY(cudaMemsetAsync(h->arrivals, 0, sizeof(unsigned) * (n - 1), s));
-        bh_bottomup_kernel<<<(unsigned)((n + BU_THREADS - 1) / BU_THREADS), BU_THREADS, 0, s>>>(
-            h->leaf, h->child, h->parent, (int)n, h->arrivals, h->sums, h->bmin, h->bmax, h->inode, h->root, h->diag);
-    }
     GB_CUDA_TRY(cudaGetLastError());
     mark(h, slot, 4, s);
-    h->launches += 5 + passes - (n >= 2 ? 0 : 1);
+    h->launches += 2 + passes;
     h->n = n;
     return GB_OK;
 }
@@ -751,21 +1037,14 @@ static int traverse(gb_bh_t *h, float4 *acc, float4 *vel, float *phi, float thet
         const int64_t warps = (nt + 31) / 32;
         const unsigned grid = (unsigned)((warps + GW_WARPS - 1) / GW_WARPS);
         if (h->groups_n != n) {
-            // Built in another traversal mode: mark the groups from the
-            // sorted keys of the same build (the topology is rewritten with
-            // identical values).
-            int *gsize = h->gsize;
-            GB_CUDA_TRY(cudaMemsetAsync(gsize, 0, sizeof(int) * n, s));
-            const int ni = (int)std::max<int64_t>(n - 1, 1);
-            if (h->key_bits == 10)
-                bh_karras_kernel<uint32_t><<<(ni + 255) / 256, 256, 0, s>>>(
-                    (const uint32_t *)h->keys[h->cur], (int)n, h->child, h->parent, gsize);
-            else
-                bh_karras_kernel<uint64_t><<<(ni + 255) / 256, 256, 0, s>>>(
-                    (const uint64_t *)h->keys[h->cur], (int)n, h->child, h->parent, gsize);
-            GB_CUDA_TRY(cudaGetLastError());
-            h->launches += 1;
-            h->groups_n = n;
+            // Built in another traversal mode: mark the groups by a second
+            // pass over the same build (identical values).
+            GB_CUDA_TRY(cudaMemsetAsync(h->gsize, 0, sizeof(int) * n, s));
+            int64_t units, groups;
+            tree_units(n, &units, &groups);
+            GB_CUDA_TRY(cudaMemsetAsync(h->tree_done, 0, sizeof(unsigned) * groups, s));
+            if (h->key_bits == 10) GB_TRY(build_tree<uint32_t>(h, nullptr, nullptr, n, true, s));
+            else GB_TRY(build_tree<uint64_t>(h, nullptr, nullptr, n, true, s));
         }
         dispatch3<GroupLaunch>(kdk, count, phi != nullptr, grid, &a, (const int *)h->gsize, phi, range, s);
     } else {

@@ -106,8 +106,8 @@ __device__ __forceinline__ GridPart cta_merge(GridPart p, GridPart *w) {
 __global__ void __launch_bounds__(GRID_THREADS)
 grid_reduce_kernel(const float4 *__restrict__ xm, const float *__restrict__ hsml, const int *__restrict__ is_star,
                    int64_t n, double min_radius, long long max_cells, GridPart *part, unsigned *ticket,
-                   GridGeom *geom, uint32_t *zero, int64_t nzero) {
-    rs_zero(zero, nzero);  // the sort's scratch
+                   GridGeom *geom, ZeroWords zero) {
+    zero_words(zero);  // the sort's scratch
     float mn0 = INFINITY, mn1 = INFINITY, mn2 = INFINITY, mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY;
     float hm = -INFINITY;
     unsigned long long cnt = 0, bad = 0;
@@ -405,8 +405,8 @@ extern "C" int gb_grid_rebuild(gb_grid_t *h, const float *xm, const float *hsml,
         if (!gsort || !cell_start) return fail(GB_EINVAL, "gsort and cell_start must not be NULL");
         const int nblk = std::max(1, std::min(h->red_blocks, (int)((n + GRID_THREADS - 1) / GRID_THREADS)));
         grid_reduce_kernel<<<nblk, GRID_THREADS, 0, s>>>((const float4 *)xm, hsml, is_star, n, h->min_radius,
-                                                        h->max_cells, h->part, h->ticket, h->geom, h->sort_scratch,
-                                                        radix_zero_words(n));
+                                                        h->max_cells, h->part, h->ticket, h->geom,
+                                                        ZeroWords{{h->sort_scratch}, {radix_zero_words(n)}});
         const unsigned g = (unsigned)((n + GRID_THREADS - 1) / GRID_THREADS);
         grid_key_kernel<<<nblk, GRID_THREADS, 0, s>>>((const float4 *)xm, is_star, n, h->geom, h->keys[0],
                                                       h->sort_scratch, h->passes);

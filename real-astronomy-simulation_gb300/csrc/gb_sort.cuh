@@ -151,10 +151,19 @@ struct RsCount {
     }
 };
 
-// Zeroes the first nz scratch words (a kernel that runs before the keys').
-__device__ __forceinline__ void rs_zero(uint32_t *scratch, int64_t nz) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nz; i += (int64_t)gridDim.x * blockDim.x)
-        scratch[i] = 0u;
+// Words that a kernel running before the keys' zeroes for the kernels behind
+// it (a memset node each would cost a launch).
+struct ZeroWords {
+    uint32_t *p[3];
+    int64_t n[3];
+};
+
+__device__ __forceinline__ void zero_words(const ZeroWords &z) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+        for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < z.n[k];
+             i += (int64_t)gridDim.x * blockDim.x)
+            z.p[k][i] = 0u;
 }
 
 // Exclusive scan of 256 values held one per thread of a 256-thread CTA.
