@@ -169,6 +169,24 @@ __device__ __noinline__ uint32_t quantise_fp64(float x, double lo, double scale,
     return __double2uint_rz(t);
 }
 
+// The Morton key of particle i.
+template <typename KeyT, int BITS>
+struct MortonKey {
+    const float4 *__restrict__ xm;
+    const BHParams *__restrict__ prm;
+
+    __device__ __forceinline__ KeyT operator()(int64_t i) const {
+        constexpr uint32_t QMAX = (1u << BITS) - 1u;
+        const float4 x = xm[i];
+        const float sh = prm->sh, sl = prm->sl;
+        uint32_t qx, qy, qz;
+        if (!cell_fp32(x.x, prm->lof[0], sh, sl, qx)) qx = quantise_fp64(x.x, prm->lo[0], prm->scale, (double)QMAX);
+        if (!cell_fp32(x.y, prm->lof[1], sh, sl, qy)) qy = quantise_fp64(x.y, prm->lo[1], prm->scale, (double)QMAX);
+        if (!cell_fp32(x.z, prm->lof[2], sh, sl, qz)) qz = quantise_fp64(x.z, prm->lo[2], prm->scale, (double)QMAX);
+        return (KeyT)interleave3<BITS>(min(qx, QMAX), min(qy, QMAX), min(qz, QMAX));
+    }
+};
+
 // Keys and, beside them, the digit counts of the sort (4 CTAs per SM share the
 // particles, so that a CTA counts many keys before it adds them up).  1M
 // particles, 30-bit keys: 11.2 us, against 35.1 us for FP64 keys alone and
@@ -178,19 +196,13 @@ __global__ void __launch_bounds__(KEY_THREADS)
 bh_morton_kernel(const float4 *__restrict__ xm, int64_t n, const BHParams *__restrict__ prm,
                  KeyT *__restrict__ keys, uint32_t *__restrict__ counts) {
     constexpr int PASSES = (3 * BITS + 7) / 8;
-    constexpr uint32_t QMAX = (1u << BITS) - 1u;
     __shared__ RsCount<PASSES> cnt;
     cnt.clear();
-    const float lo0 = prm->lof[0], lo1 = prm->lof[1], lo2 = prm->lof[2], sh = prm->sh, sl = prm->sl;
+    const MortonKey<KeyT, BITS> key{xm, prm};
     for (int64_t i = (int64_t)blockIdx.x * KEY_THREADS + threadIdx.x; i < n; i += (int64_t)gridDim.x * KEY_THREADS) {
-        const float4 x = xm[i];
-        uint32_t qx, qy, qz;
-        if (!cell_fp32(x.x, lo0, sh, sl, qx)) qx = quantise_fp64(x.x, prm->lo[0], prm->scale, (double)QMAX);
-        if (!cell_fp32(x.y, lo1, sh, sl, qy)) qy = quantise_fp64(x.y, prm->lo[1], prm->scale, (double)QMAX);
-        if (!cell_fp32(x.z, lo2, sh, sl, qz)) qz = quantise_fp64(x.z, prm->lo[2], prm->scale, (double)QMAX);
-        const KeyT key = (KeyT)interleave3<BITS>(min(qx, QMAX), min(qy, QMAX), min(qz, QMAX));
-        keys[i] = key;
-        cnt.add(key, PASSES);
+        const KeyT k = key(i);
+        keys[i] = k;
+        cnt.add(k, PASSES);
     }
     cnt.flush(counts, PASSES);
 }
@@ -913,11 +925,12 @@ static int build_impl(gb_bh_t *h, float4 *xm, float4 *vel, const float4 *acc, in
     mark(h, slot, 0, s);
     const int nblk = std::max(1, std::min(h->bbox_blocks, (int)((n + BBOX_THREADS - 1) / BBOX_THREADS)));
     // The sort's scratch, the tree's finished units and the group walk's marks.
-    const bool groups = h->tpl == 3;
+    constexpr int passes = (3 * BITS + 7) / 8;
+    const bool groups = h->tpl == 3, small = radix_small(n, passes);
     int64_t units, ngroups;
     tree_units(n, &units, &ngroups);
     const ZeroWords zero = {{h->sort_scratch, h->tree_done, (uint32_t *)h->gsize},
-                            {radix_zero_words(n), ngroups, groups ? n : 0}};
+                            {small ? 0 : radix_zero_words(n), ngroups, groups ? n : 0}};
     if (kdk)
         bh_bbox_kernel<true><<<nblk, BBOX_THREADS, 0, s>>>(xm, vel, acc, n, 0.5f * dt, dt, h->bbox_part, h->ticket,
                                                            h->prm, BITS, zero, h->diag);
@@ -925,18 +938,22 @@ static int build_impl(gb_bh_t *h, float4 *xm, float4 *vel, const float4 *acc, in
         bh_bbox_kernel<false><<<nblk, BBOX_THREADS, 0, s>>>(xm, nullptr, nullptr, n, 0.f, 0.f, h->bbox_part,
                                                             h->ticket, h->prm, BITS, zero, h->diag);
     KeyT *kk[2] = {(KeyT *)h->keys[0], (KeyT *)h->keys[1]};
-    const unsigned gk = std::min((unsigned)(h->sms * 4), (unsigned)((n + KEY_THREADS - 1) / KEY_THREADS));
-    bh_morton_kernel<KeyT, BITS><<<gk, KEY_THREADS, 0, s>>>(xm, n, h->prm, kk[0], h->sort_scratch);
-    mark(h, slot, 1, s);
-    const int passes = (3 * BITS + 7) / 8;
-    h->cur = radix_sort_counted<KeyT>(kk, h->vals, n, passes, h->sort_scratch, h->diag, s);
+    if (small) {
+        mark(h, slot, 1, s);
+        h->cur = radix_sort_small<KeyT>(MortonKey<KeyT, BITS>{xm, h->prm}, kk, h->vals, n, s);
+    } else {
+        const unsigned gk = std::min((unsigned)(h->sms * 4), (unsigned)((n + KEY_THREADS - 1) / KEY_THREADS));
+        bh_morton_kernel<KeyT, BITS><<<gk, KEY_THREADS, 0, s>>>(xm, n, h->prm, kk[0], h->sort_scratch);
+        mark(h, slot, 1, s);
+        h->cur = radix_sort_counted<KeyT>(kk, h->vals, n, passes, h->sort_scratch, h->diag, s);
+    }
     mark(h, slot, 2, s);
     // The group walk's groups are marked when the handle walks groups.
     GB_TRY(build_tree<KeyT>(h, xm, h->vals[h->cur], n, groups, s));
     mark(h, slot, 3, s);
     GB_CUDA_TRY(cudaGetLastError());
     mark(h, slot, 4, s);
-    h->launches += 2 + passes;
+    h->launches += small ? 1 + radix_small_launches(n) : 2 + passes;
     h->n = n;
     return GB_OK;
 }

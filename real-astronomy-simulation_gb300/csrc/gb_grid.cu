@@ -215,36 +215,41 @@ __device__ __noinline__ uint32_t cell_fp64(float x, double lo, double cell, int 
     return (uint32_t)(v < 0 ? 0 : (v > dim - 1 ? dim - 1 : v));
 }
 
-// Cell key of every particle, and the digit counts of the sort; stars and
-// inactive rebuilds get n_cells (or 0), which sorts after every gas key.
-// 1M particles: 11.4 us, against 67.7 us with FP64 divisions and 13.7 us for
-// a kernel that counted the digits.
+// Cell key of particle i; stars and inactive rebuilds get n_cells (or 0),
+// which sorts after every gas key.
+struct CellKey {
+    const float4 *__restrict__ xm;
+    const int *__restrict__ is_star;
+    const GridGeom *__restrict__ geom;
+
+    __device__ __forceinline__ uint32_t operator()(int64_t i) const {
+        const GridGeom &g = *geom;
+        if (!g.active) return 0u;
+        if (is_star && __ldg(is_star + i) != 0) return (uint32_t)g.n_cells;
+        const float4 p = __ldg(xm + i);
+        const float c[3] = {p.x, p.y, p.z}, ih = g.ih, il = g.il;
+        const int dim[3] = {g.nx, g.ny, g.nz};
+        uint32_t q[3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            if (!cell_fp32(c[a], g.lof[a], ih, il, q[a])) q[a] = cell_fp64(c[a], g.lo[a], g.cell, dim[a]);
+            q[a] = min(q[a], (uint32_t)(dim[a] - 1));
+        }
+        return (q[0] * (uint32_t)dim[1] + q[1]) * (uint32_t)dim[2] + q[2];
+    }
+};
+
+// All keys, and the digit counts of the sort.  1M particles: 11.4 us, against
+// 67.7 us with FP64 divisions and 13.7 us for a kernel that counted the digits.
 __global__ void __launch_bounds__(GRID_THREADS)
-grid_key_kernel(const float4 *__restrict__ xm, const int *__restrict__ is_star, int64_t n,
-                const GridGeom *__restrict__ geom, uint32_t *keys, uint32_t *counts, int passes) {
+grid_key_kernel(CellKey key, int64_t n, uint32_t *keys, uint32_t *counts, int passes) {
     __shared__ RsCount<4> cnt;
     cnt.clear();
-    const GridGeom &g = *geom;
-    const bool active = g.active;
-    const int dim[3] = {g.nx, g.ny, g.nz};
-    const float lof[3] = {g.lof[0], g.lof[1], g.lof[2]}, ih = g.ih, il = g.il;
-    const uint32_t none = active ? (uint32_t)g.n_cells : 0u;
     for (int64_t i = (int64_t)blockIdx.x * GRID_THREADS + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * GRID_THREADS) {
-        uint32_t key = none;
-        if (active && !(is_star && __ldg(is_star + i) != 0)) {
-            const float4 p = __ldg(xm + i);
-            const float c[3] = {p.x, p.y, p.z};
-            uint32_t q[3];
-#pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                if (!cell_fp32(c[a], lof[a], ih, il, q[a])) q[a] = cell_fp64(c[a], g.lo[a], g.cell, dim[a]);
-                q[a] = min(q[a], (uint32_t)(dim[a] - 1));
-            }
-            key = (q[0] * (uint32_t)dim[1] + q[1]) * (uint32_t)dim[2] + q[2];
-        }
-        keys[i] = key;
-        cnt.add(key, passes);
+        const uint32_t k = key(i);
+        keys[i] = k;
+        cnt.add(k, passes);
     }
     cnt.flush(counts, passes);
 }
@@ -254,19 +259,6 @@ __global__ void grid_gsort_kernel(const uint32_t *__restrict__ vals, int64_t n, 
     const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= n || !geom->active) return;
     gsort[p] = p < geom->ngas ? (int)vals[p] : 0;
-}
-
-// First index in [0, n) with key >= c, found by a warp: 32 probes per step.
-__device__ __forceinline__ long long warp_lower_bound(const uint32_t *__restrict__ keys, long long n, long long c) {
-    const int lane = threadIdx.x & 31;
-    long long lo = 0, hi = n;
-    while (lo < hi) {
-        const long long step = (hi - lo + 32) / 33, at = lo + (lane + 1) * step - 1;
-        const int below = __popc(__ballot_sync(0xffffffffu, at < hi && (long long)__ldg(keys + at) < c));
-        hi = below < 32 ? min(hi, lo + (below + 1) * step - 1) : hi;
-        lo += below * step;
-    }
-    return lo;
 }
 
 // cell_start[c] = lower bound of c in the sorted gas keys (c <= n_cells);
@@ -296,7 +288,7 @@ grid_start_kernel(const uint32_t *__restrict__ keys, const GridGeom *__restrict_
     if (c0 <= nc) {
         if (tid < 64) {
             const int k = tid >> 5;
-            const long long r = warp_lower_bound(keys, ng, c0 + k * START_CELLS);
+            const long long r = warp_bound(keys, ng, (uint32_t)(c0 + k * START_CELLS));
             if ((tid & 31) == 0) range[k] = (int)r;
         }
         __syncthreads();
@@ -404,18 +396,24 @@ extern "C" int gb_grid_rebuild(gb_grid_t *h, const float *xm, const float *hsml,
         if (!hsml) return fail(GB_EINVAL, "hsml is NULL");
         if (!gsort || !cell_start) return fail(GB_EINVAL, "gsort and cell_start must not be NULL");
         const int nblk = std::max(1, std::min(h->red_blocks, (int)((n + GRID_THREADS - 1) / GRID_THREADS)));
+        const bool small = radix_small(n, h->passes);
         grid_reduce_kernel<<<nblk, GRID_THREADS, 0, s>>>((const float4 *)xm, hsml, is_star, n, h->min_radius,
                                                         h->max_cells, h->part, h->ticket, h->geom,
-                                                        ZeroWords{{h->sort_scratch}, {radix_zero_words(n)}});
+                                                        ZeroWords{{h->sort_scratch}, {small ? 0 : radix_zero_words(n)}});
         const unsigned g = (unsigned)((n + GRID_THREADS - 1) / GRID_THREADS);
-        grid_key_kernel<<<nblk, GRID_THREADS, 0, s>>>((const float4 *)xm, is_star, n, h->geom, h->keys[0],
-                                                      h->sort_scratch, h->passes);
-        const int cur = radix_sort_counted<uint32_t>(h->keys, h->vals, n, h->passes, h->sort_scratch, h->diag, s);
+        const CellKey key{(const float4 *)xm, is_star, h->geom};
+        int cur = 0;
+        if (small) {
+            cur = radix_sort_small<uint32_t>(key, h->keys, h->vals, n, s);
+        } else {
+            grid_key_kernel<<<nblk, GRID_THREADS, 0, s>>>(key, n, h->keys[0], h->sort_scratch, h->passes);
+            cur = radix_sort_counted<uint32_t>(h->keys, h->vals, n, h->passes, h->sort_scratch, h->diag, s);
+        }
         grid_gsort_kernel<<<g, GRID_THREADS, 0, s>>>(h->vals[cur], n, h->geom, gsort);
         const unsigned gc = (unsigned)((h->max_cells + START_CELLS) / START_CELLS);
         grid_start_kernel<<<gc, GRID_THREADS, 0, s>>>(h->keys[cur], h->geom, h->max_cells, cell_start);
         GB_CUDA_TRY(cudaGetLastError());
-        h->launches += 4 + h->passes;
+        h->launches += small ? 3 + radix_small_launches(n) : 4 + h->passes;
     }
     if (info) {
         GridGeom g;

@@ -16,6 +16,10 @@
 // already running and publishes its count without waiting itself.  Each wait
 // is bounded: after RS_SPIN_LIMIT polls the CTA counts DIAG_WAIT_TIMEOUT and
 // goes on with the prefix it has (its scatter still stays inside [0, n)).
+//
+// Smaller sorts (radix_small) take up to three kernels instead: blocks of 1,024
+// keys are made and sorted in shared memory, then every key finds its place
+// among a group of blocks, and among the groups, by binary search.
 #pragma once
 
 #include <algorithm>
@@ -286,6 +290,227 @@ rs_onesweep_kernel(const KeyT *__restrict__ kin, const uint32_t *__restrict__ vi
             atomicAdd(diag + DIAG_BAD_TREE, 1ull);
         }
     }
+}
+
+// ------------------------------------------------------------ small sorts
+// First kernel: a CTA makes 1,024 keys (src(i): the key of index i) and sorts
+// them with their indices: 32 at a time by a bitonic network in each warp,
+// then five rounds that merge neighbouring runs, a key's place in its pair of
+// runs being its place in its own plus the keys before it in the other
+// (binary search; equal keys of the earlier run come first, so the sort is
+// stable).
+constexpr int SS_BLOCK = 1024;
+
+template <typename KeyT>
+__device__ __forceinline__ int ss_count(const KeyT *run, int len, KeyT key, bool equal_too) {
+    int at = 0;  // len is a power of two; at < len before the last comparison
+    for (int step = len >> 1; step > 0; step >>= 1) {
+        const KeyT x = run[at + step - 1];
+        if (x < key || (equal_too && x == key)) at += step;
+    }
+    const KeyT x = run[at];
+    return at + (x < key || (equal_too && x == key));
+}
+
+template <typename KeyT, typename Source>
+__global__ void __launch_bounds__(SS_BLOCK)
+ss_block_kernel(Source src, int n, KeyT *__restrict__ kout, uint32_t *__restrict__ vout) {
+    __shared__ KeyT sk[2][SS_BLOCK];
+    __shared__ uint32_t sv[2][SS_BLOCK];
+    const int tid = threadIdx.x, lane = tid & 31, g = blockIdx.x * SS_BLOCK + tid;
+    KeyT key = g < n ? src(g) : ~(KeyT)0;  // above every key: the last ones
+    uint32_t val = (uint32_t)g;
+#pragma unroll
+    for (int k = 2; k <= 32; k <<= 1)
+#pragma unroll
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            const KeyT ok = __shfl_xor_sync(0xffffffffu, key, j);
+            const uint32_t ov = __shfl_xor_sync(0xffffffffu, val, j);
+            const bool less = ok < key || (ok == key && ov < val);        // the other one comes first
+            const bool want_first = ((lane & k) == 0) == ((lane & j) == 0);  // k = 32: ascending
+            if (less == want_first) {
+                key = ok;
+                val = ov;
+            }
+        }
+    int buf = 0;
+    sk[0][tid] = key;
+    sv[0][tid] = val;
+    __syncthreads();
+#pragma unroll
+    for (int len = 32; len < SS_BLOCK; len <<= 1) {
+        const int other = (tid & ~(len - 1)) ^ len;
+        const int to = (tid & ~(2 * len - 1)) + (tid & (len - 1)) + ss_count(sk[buf] + other, len, key, other < tid);
+        sk[buf ^ 1][to] = key;
+        sv[buf ^ 1][to] = val;
+        buf ^= 1;
+        __syncthreads();
+        key = sk[buf][tid];
+        val = sv[buf][tid];
+    }
+    if (g < n) {
+        kout[g] = key;
+        vout[g] = val;
+    }
+}
+
+// First index in [0, n) with key >= c (above: > c), found by a warp: 32 probes
+// per step.
+template <typename KeyT, typename IndexT>
+__device__ __forceinline__ IndexT warp_bound(const KeyT *__restrict__ keys, IndexT n, KeyT c, bool above = false) {
+    const int lane = threadIdx.x & 31;
+    IndexT lo = 0, hi = n;
+    while (lo < hi) {
+        const IndexT step = (hi - lo + 32) / 33, at = lo + (lane + 1) * step - 1;
+        const KeyT x = at < hi ? __ldg(keys + at) : (KeyT)0;
+        const int below = __popc(__ballot_sync(0xffffffffu, at < hi && (x < c || (above && x == c))));
+        hi = below < 32 ? min(hi, lo + (below + 1) * step - 1) : hi;
+        lo += below * step;
+    }
+    return lo;
+}
+
+// Second kernel: a group of neighbouring sorted blocks becomes one.  The place
+// of a key is its place in its block plus the keys before it in every other
+// block of the group (those of earlier blocks where equal).  A CTA takes
+// SS_KEYS consecutive keys of a block and passes over the group's blocks,
+// SS_SIDE of them at a time in shared memory, whose searches run side by side;
+// a warp's keys are neighbours, so they read the same or neighbouring words.
+constexpr int SS_KEYS = 256;
+constexpr int SS_SIDE = 4;
+
+template <typename KeyT>
+__global__ void __launch_bounds__(SS_KEYS)
+ss_group_kernel(const KeyT *__restrict__ kin, const uint32_t *__restrict__ vin, int n, int group,
+                KeyT *__restrict__ kout, uint32_t *__restrict__ vout) {
+    __shared__ KeyT blk[SS_SIDE][SS_BLOCK];
+    const int tid = threadIdx.x, g = blockIdx.x * SS_KEYS + tid, mine = blockIdx.x / (SS_BLOCK / SS_KEYS);
+    const int first = mine / group * group, end = min(first + group, (n + SS_BLOCK - 1) / SS_BLOCK);
+    const KeyT key = g < n ? __ldg(kin + g) : ~(KeyT)0;
+    int place = first * SS_BLOCK + (g - mine * SS_BLOCK);
+    for (int b0 = first; b0 < end; b0 += SS_SIDE) {
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < SS_SIDE * SS_BLOCK / SS_KEYS; ++q) {
+            const int i = q * SS_KEYS + tid, x = b0 * SS_BLOCK + i;
+            (&blk[0][0])[i] = x < min(n, end * SS_BLOCK) ? __ldg(kin + x) : ~(KeyT)0;
+        }
+        __syncthreads();
+        int at[SS_SIDE];
+#pragma unroll
+        for (int q = 0; q < SS_SIDE; ++q) at[q] = 0;
+#pragma unroll
+        for (int step = SS_BLOCK >> 1; step > 0; step >>= 1)
+#pragma unroll
+            for (int q = 0; q < SS_SIDE; ++q) {
+                const KeyT x = blk[q][at[q] + step - 1];
+                if (x < key || (b0 + q < mine && x == key)) at[q] += step;
+            }
+#pragma unroll
+        for (int q = 0; q < SS_SIDE; ++q) {
+            const KeyT x = blk[q][at[q]];
+            if (x < key || (b0 + q < mine && x == key)) ++at[q];
+            if (b0 + q != mine) place += at[q];  // past the group's end no key is below ~0
+        }
+    }
+    if (g < n && place < n) {
+        kout[place] = key;
+        vout[place] = __ldg(vin + g);
+    }
+}
+
+// Third kernel: all groups, sorted blocks of len keys, become one.  The places
+// of a CTA's first and last key bound its searches in another block (a 32-way
+// search by a warp each), which are short and read neighbouring words of L1.
+constexpr int SS_MAX_GROUPS = 16;
+
+template <typename KeyT>
+__global__ void __launch_bounds__(SS_KEYS)
+ss_merge_kernel(const KeyT *__restrict__ kin, const uint32_t *__restrict__ vin, int n, int len,
+                KeyT *__restrict__ kout, uint32_t *__restrict__ vout) {
+    __shared__ int from[SS_MAX_GROUPS], size[SS_MAX_GROUPS];  // the window in each block
+    const int tid = threadIdx.x, wid = tid >> 5, g0 = blockIdx.x * SS_KEYS, g = g0 + tid;
+    const int mine = g0 / len, blocks = (n + len - 1) / len;
+    const KeyT key = g < n ? __ldg(kin + g) : ~(KeyT)0;
+    const KeyT kmin = __ldg(kin + g0), kmax = __ldg(kin + min(g0 + SS_KEYS, n) - 1);
+    for (int t = wid; t < blocks; t += SS_KEYS / 32) {
+        const int start = t * len, cnt = min(len, n - start);
+        int lo = 0, m = 0;
+        if (t != mine) {
+            lo = warp_bound(kin + start, cnt, kmin);
+            m = warp_bound(kin + start + lo, cnt - lo, kmax, true);
+        }
+        if ((tid & 31) == 0) {
+            from[t] = start + lo;
+            size[t] = m;
+        }
+    }
+    __syncthreads();
+    int place = g - mine * len;
+    for (int t0 = 0; t0 < blocks; t0 += SS_SIDE) {
+        int at[SS_SIDE], m[SS_SIDE], most = 0;
+        const KeyT *win[SS_SIDE];
+#pragma unroll
+        for (int q = 0; q < SS_SIDE; ++q) {
+            const bool in = t0 + q < blocks;
+            const int f = in ? from[t0 + q] : 0;
+            win[q] = kin + f;
+            m[q] = in ? size[t0 + q] : 0;
+            most = max(most, m[q]);
+            at[q] = 0;
+            if (in && t0 + q != mine) place += f - (t0 + q) * len;
+        }
+        for (int step = most > 0 ? 1 << (31 - __clz(most)) : 0; step > 0; step >>= 1)
+#pragma unroll
+            for (int q = 0; q < SS_SIDE; ++q)
+                if (at[q] + step <= m[q]) {
+                    const KeyT x = __ldg(win[q] + at[q] + step - 1);
+                    if (x < key || (t0 + q < mine && x == key)) at[q] += step;
+                }
+#pragma unroll
+        for (int q = 0; q < SS_SIDE; ++q) place += at[q];
+    }
+    if (g < n && place < n) {
+        kout[place] = key;
+        vout[place] = __ldg(vin + g);
+    }
+}
+
+// Whether a sort of n keys in `passes` digits takes these kernels.  Bounding
+// box, keys and sort on the disk (us, with a kernel per digit in brackets),
+// 63-bit keys (8 digits): 1,000: 19 (72); 10,000: 28 (94); 33,000: 40 (96);
+// 100,000: 54 (104); 131,072: 58 (114); 200,000: 93 (121); 262,144: 108 (123).
+// 30-bit keys (4): 10,000: 24 (52); 33,000: 36 (56); 100,000: 49 (62); 131,072:
+// 51 (64); 200,000: 79 (72).  A kernel per digit costs 7 to 9 us whatever its
+// size, mostly launch, look-back and ranking latency; these grow with the
+// number of blocks each key is compared with.  Groups of 32: 63 at 100,000;
+// blocks' windows instead of whole blocks in the second kernel too: 36 at
+// 10,000, 65 at 100,000; one stage over all blocks: 98 at 100,000.
+constexpr int64_t SS_ONE_N = 32 * SS_BLOCK;  // one group
+constexpr int64_t SS_GROUP = 16;             // blocks per group above
+constexpr int64_t SS_MAX_N8 = 262144, SS_MAX_N4 = 131072, SS_MAX_N3 = 65536;
+static_assert(SS_MAX_N8 <= SS_MAX_GROUPS * SS_GROUP * SS_BLOCK, "a window per group");
+inline bool radix_small(int64_t n, int passes) {
+    return n <= (passes > 4 ? SS_MAX_N8 : passes == 4 ? SS_MAX_N4 : SS_MAX_N3);
+}
+
+// Kernels of such a sort.
+inline int radix_small_launches(int64_t n) { return n <= SS_BLOCK ? 1 : n <= SS_ONE_N ? 2 : 3; }
+
+// Sorts the keys src(0 .. n - 1) with their indices; returns the index of the
+// pair of k and v that holds the result.
+template <typename KeyT, typename Source>
+static int radix_sort_small(const Source &src, KeyT *k[2], uint32_t *v[2], int64_t n, cudaStream_t s) {
+    const int launches = radix_small_launches(n);
+    const unsigned gr = (unsigned)((n + SS_KEYS - 1) / SS_KEYS);
+    ss_block_kernel<KeyT, Source><<<(unsigned)((n + SS_BLOCK - 1) / SS_BLOCK), SS_BLOCK, 0, s>>>(src, (int)n, k[0],
+                                                                                               v[0]);
+    if (launches > 1)
+        ss_group_kernel<KeyT><<<gr, SS_KEYS, 0, s>>>(k[0], v[0], (int)n, launches == 2 ? 32 : (int)SS_GROUP, k[1],
+                                                     v[1]);
+    if (launches > 2)
+        ss_merge_kernel<KeyT><<<gr, SS_KEYS, 0, s>>>(k[1], v[1], (int)n, (int)(SS_GROUP * SS_BLOCK), k[0], v[0]);
+    return launches == 2 ? 1 : 0;
 }
 
 // Scratch words that are zero when the kernel that makes the keys starts:

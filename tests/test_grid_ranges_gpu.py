@@ -13,7 +13,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("n,spread", [(1, "line"), (33, "line"), (255, "line"), (256, "line"), (257, "line"), (3000, "line"),
-                                      (3000, "point"), (40000, "point"), (40000, "two"), (100003, "line")])
+                                      (3000, "point"), (40000, "point"), (40000, "two"), (65536, "line"), (65537, "two"),
+                                      (100003, "line")])
 def test_cell_start_ranges(cuda_dev, orc, n, spread):
     """Keys spread over the cells, all in one cell, or in the first and the
     last one (one CTA then holds all keys, or almost all hold none)."""
