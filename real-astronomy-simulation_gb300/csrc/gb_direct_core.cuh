@@ -160,6 +160,13 @@ static inline int64_t sym_bands(int64_t nt, int64_t budget, std::vector<int64_t>
     return std::max(max_pairs, pairs);
 }
 
+// Whether the slots of a symmetric pass in tiles of `tile` particles and Q
+// slices fit one band of band_bytes.
+static inline bool sym_one_band(int64_t n, int tile, int Q, int64_t band_bytes) {
+    const int64_t nt = (n + tile - 1) / tile;
+    return nt * (nt + 1) / 2 <= band_bytes / ((int64_t)sizeof(float4) * tile * (Q + 1));
+}
+
 static inline int64_t host_sym_base(int64_t I, int64_t nt) { return I * nt - I * (I - 1) / 2; }
 
 // Symmetric (tile-pair) scratch above this size is not used: the callers

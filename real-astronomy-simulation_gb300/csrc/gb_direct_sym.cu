@@ -44,13 +44,24 @@ constexpr int DS_ACC = 0, DS_KDK = 1, DS_PHI = 2;
 // registers at 6) it halves the per-source overhead per pair (staging, the
 // shared-memory sum and its 6 scalar adds), and with up to 8 source slices
 // per tile pair its units stay short enough for small systems too.
-template <int H>
+template <int H, int T>
 struct DsShape {
-    static constexpr int WARPS = 8 / H, WT = 64 * H, MIN_CTAS = H == 4 ? 8 : 6;
-    static constexpr int QMAX = 16 / WARPS;  // each warp of a round takes its own source group
-    static_assert(WARPS * WT == DS_T, "a CTA's warps cover one tile");
+    static constexpr int WT = 64 * H, WARPS = T / WT, MIN_CTAS = H == 4 ? 8 : 12;
+    static constexpr int QMAX = T / 32 / WARPS;  // each warp of a round takes its own source group
+    static_assert(WARPS * WT == T, "a CTA's warps cover one tile");
 };
 constexpr int DS_H = 4;
+// Small systems (one system of at most DS_SMALL_N particles): tiles of 256, 4
+// targets per lane, four source slices per tile pair.  The time is one unit's
+// serial length: a tile pair of 512 in four slices keeps a warp busy for 128
+// sources x 8 targets a lane, one of 256 for 64 x 4.  Up to 6,144 particles
+// (300 tile pairs, 1,200 units) the small units still run in one wave, so each
+// CTA takes the unit of its index and the counter with its memset is left out.
+// Microseconds per KDK step, tiles of 512 with the counter / 512 without / 256:
+// 1,000: 18.5 / 14.7 / 11.6; 4,096: 18.5 / 15.7 / 14.6; 6,144: - / 26.2 / 21.1;
+// past the wave the twice as many slots cost more: 8,000: - / 32.9 / 37.2.
+constexpr int DS_SMALL_T = 256, DS_SMALL_H = 2, DS_SMALL_Q = 4;
+constexpr int64_t DS_SMALL_N = 6144;
 
 struct DsArgs {
     const float4 *__restrict__ xm;
@@ -58,7 +69,7 @@ struct DsArgs {
     const float4 *__restrict__ acc;
     float4 *__restrict__ rowpart;  // NU x DS_T (one row slot per unit)
     float4 *__restrict__ colpart;  // tile pairs x DS_T
-    unsigned long long *counter;   // zero at launch
+    unsigned long long *counter;   // zero at launch; NULL: one unit per CTA
     int64_t n, nt, NU;             // one system: particles, tiles; units in all
     int64_t p0;                    // one system: first tile pair of the band
     // Many systems (BATCH): nsys + 1 particle offsets, unit bases and
@@ -104,7 +115,7 @@ __device__ __forceinline__ void ds_round(const float4 *__restrict__ sxm, float4 
             if (DIAG) {  // a zero inv zeroes the pair's force and potential terms
                 float c0, c1;
                 unpack2(inv, c0, c1);
-                const int t0 = DsShape<H>::WT * wib + 64 * h + lane;
+                const int t0 = 64 * H * wib + 64 * h + lane;
                 c0 = t0 < jj ? c0 : 0.f;
                 c1 = t0 + 32 < jj ? c1 : 0.f;
                 inv = pack2(c0, c1);
@@ -164,7 +175,7 @@ __device__ __forceinline__ void ds_round_phi(const float4 *__restrict__ sxm, flo
             if (DIAG) {
                 float c0, c1;
                 unpack2(inv, c0, c1);
-                const int t0 = DsShape<H>::WT * wib + 64 * h + lane;
+                const int t0 = 64 * H * wib + 64 * h + lane;
                 c0 = t0 < jj ? c0 : 0.f;
                 c1 = t0 + 32 < jj ? c1 : 0.f;
                 inv = pack2(c0, c1);
@@ -183,10 +194,11 @@ __device__ __forceinline__ void ds_round_phi(const float4 *__restrict__ sxm, flo
 
 // PHI (one system, MODE DS_ACC or DS_KDK): the pass also returns the
 // potential sums of its positions, in the slots' .w.
-template <int Q, int MODE, bool BATCH, int H, bool PHI>
-__global__ void __launch_bounds__(DsShape<H>::WARPS * 32, DsShape<H>::MIN_CTAS) direct_sym_kernel(DsArgs a) {
-    constexpr int G = 16 / Q, SPAN = G * 32;
-    constexpr int WARPS = DsShape<H>::WARPS, WT = DsShape<H>::WT;
+template <int Q, int MODE, bool BATCH, int H, bool PHI, int T>
+__global__ void __launch_bounds__(DsShape<H, T>::WARPS * 32, DsShape<H, T>::MIN_CTAS) direct_sym_kernel(DsArgs a) {
+    constexpr int DS_T = T;
+    constexpr int G = DS_T / 32 / Q, SPAN = G * 32;
+    constexpr int WARPS = DsShape<H, T>::WARPS, WT = DsShape<H, T>::WT;
     static_assert(G >= WARPS, "each warp of a round takes its own source group");
     __shared__ float4 sxm[DS_T], sacc[DS_T];
     // The unit and, for a batch, its system's offset, size, local unit and
@@ -195,10 +207,13 @@ __global__ void __launch_bounds__(DsShape<H>::WARPS * 32, DsShape<H>::MIN_CTAS) 
     __shared__ int s_gend, s_ntgt;  // source groups and targets of the unit that hold particles
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, tid = threadIdx.x;
     const f2 EPS2 = pack2(a.eps2, a.eps2);
+    if (tid == 0) s_unit = -1;
     for (;;) {
         __syncthreads();  // the previous unit is done with the shared state
         if (tid == 0) {
-            const long long u = (long long)atomicAdd(a.counter, 1ull);
+            const long long u = a.counter     ? (long long)atomicAdd(a.counter, 1ull)
+                                : s_unit < 0 ? (long long)blockIdx.x
+                                             : (long long)a.NU;
             s_unit = u;
             if (BATCH && u < a.NU) {
                 const int sy = find_base(a.ubase, a.nsys, u);
@@ -338,8 +353,9 @@ constexpr int DS_FIX_WARPS = 8;
 // PHI: the slots also carry potential sums in .w (force pass with the
 // potential); the particle's sum is written to phi (without G) beside its
 // acceleration.
-template <int MODE, bool KAHAN, bool BATCH, bool PHI>
+template <int MODE, bool KAHAN, bool BATCH, bool PHI, int TILE>
 __global__ void __launch_bounds__(DS_FIX_WARPS * 32) direct_sym_fixup_kernel(DsFix f) {
+    constexpr int DS_T = TILE;
     __shared__ float4 part[DS_FIX_WARPS][32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     int64_t o = 0, n_s = f.n, nt = f.nt, li0 = f.Ib * DS_T + (int64_t)blockIdx.x * 32, ub = 0, cb = 0;
@@ -421,44 +437,56 @@ __global__ void __launch_bounds__(DS_FIX_WARPS * 32) direct_sym_fixup_kernel(DsF
     kdk_writeback(f.xm, f.vel, f.acc, i, an, f.h, f.dt);
 }
 
-template <int MODE, bool BATCH, int H, bool PHI>
+template <int MODE, bool BATCH, bool PHI>
 static void launch_force(int Q, unsigned grid, const DsArgs &a, cudaStream_t s) {
-    const unsigned b = DsShape<H>::WARPS * 32;
-    if (Q == 1) direct_sym_kernel<1, MODE, BATCH, H, PHI><<<grid, b, 0, s>>>(a);
-    else if (Q == 2) direct_sym_kernel<2, MODE, BATCH, H, PHI><<<grid, b, 0, s>>>(a);
-    else if (Q == 4) direct_sym_kernel<4, MODE, BATCH, H, PHI><<<grid, b, 0, s>>>(a);
-    else direct_sym_kernel<8, MODE, BATCH, H, PHI><<<grid, b, 0, s>>>(a);
+    const unsigned b = DsShape<DS_H, DS_T>::WARPS * 32;
+    if (Q == 1) direct_sym_kernel<1, MODE, BATCH, DS_H, PHI, DS_T><<<grid, b, 0, s>>>(a);
+    else if (Q == 2) direct_sym_kernel<2, MODE, BATCH, DS_H, PHI, DS_T><<<grid, b, 0, s>>>(a);
+    else if (Q == 4) direct_sym_kernel<4, MODE, BATCH, DS_H, PHI, DS_T><<<grid, b, 0, s>>>(a);
+    else direct_sym_kernel<8, MODE, BATCH, DS_H, PHI, DS_T><<<grid, b, 0, s>>>(a);
+}
+
+template <int MODE, bool BATCH, bool PHI, int T>
+static void launch_fixup(bool kahan, unsigned fgrid, const DsFix &f, cudaStream_t s) {
+    if (kahan) direct_sym_fixup_kernel<MODE, true, BATCH, PHI, T><<<fgrid, DS_FIX_WARPS * 32, 0, s>>>(f);
+    else direct_sym_fixup_kernel<MODE, false, BATCH, PHI, T><<<fgrid, DS_FIX_WARPS * 32, 0, s>>>(f);
 }
 
 template <int MODE, bool BATCH, bool PHI>
-static void launch_mode(int Q, bool kahan, unsigned grid, unsigned fgrid, const DsArgs &a, const DsFix &f,
+static void launch_mode(int tile, int Q, bool kahan, unsigned grid, unsigned fgrid, const DsArgs &a, const DsFix &f,
                         cudaStream_t s) {
-    launch_force<MODE, BATCH, DS_H, PHI>(Q, grid, a, s);
-    if (kahan) direct_sym_fixup_kernel<MODE, true, BATCH, PHI><<<fgrid, DS_FIX_WARPS * 32, 0, s>>>(f);
-    else direct_sym_fixup_kernel<MODE, false, BATCH, PHI><<<fgrid, DS_FIX_WARPS * 32, 0, s>>>(f);
+    if constexpr (!BATCH) {
+        if (tile == DS_SMALL_T) {
+            direct_sym_kernel<DS_SMALL_Q, MODE, false, DS_SMALL_H, PHI, DS_SMALL_T>
+                <<<grid, DsShape<DS_SMALL_H, DS_SMALL_T>::WARPS * 32, 0, s>>>(a);
+            return launch_fixup<MODE, false, PHI, DS_SMALL_T>(kahan, fgrid, f, s);
+        }
+    }
+    launch_force<MODE, BATCH, PHI>(Q, grid, a, s);
+    launch_fixup<MODE, BATCH, PHI, DS_T>(kahan, fgrid, f, s);
 }
 
 // mode: DS_ACC, DS_KDK or (one system) DS_PHI; phi (one system, DS_ACC or
 // DS_KDK): the force pass also writes the potential sums.
 template <bool BATCH>
-static void launch_pass(int mode, bool phi, int Q, bool kahan, unsigned grid, unsigned fgrid, const DsArgs &a,
+static void launch_pass(int mode, bool phi, int tile, int Q, bool kahan, unsigned grid, unsigned fgrid, const DsArgs &a,
                         const DsFix &f, cudaStream_t s) {
     if constexpr (!BATCH) {
-        if (phi && mode == DS_KDK) return launch_mode<DS_KDK, false, true>(Q, kahan, grid, fgrid, a, f, s);
-        if (phi && mode == DS_ACC) return launch_mode<DS_ACC, false, true>(Q, kahan, grid, fgrid, a, f, s);
+        if (phi && mode == DS_KDK) return launch_mode<DS_KDK, false, true>(tile, Q, kahan, grid, fgrid, a, f, s);
+        if (phi && mode == DS_ACC) return launch_mode<DS_ACC, false, true>(tile, Q, kahan, grid, fgrid, a, f, s);
     }
-    if (mode == DS_KDK) launch_mode<DS_KDK, BATCH, false>(Q, kahan, grid, fgrid, a, f, s);
-    else if (mode == DS_ACC) launch_mode<DS_ACC, BATCH, false>(Q, kahan, grid, fgrid, a, f, s);
-    else if constexpr (!BATCH) launch_mode<DS_PHI, BATCH, false>(Q, kahan, grid, fgrid, a, f, s);
+    if (mode == DS_KDK) launch_mode<DS_KDK, BATCH, false>(tile, Q, kahan, grid, fgrid, a, f, s);
+    else if (mode == DS_ACC) launch_mode<DS_ACC, BATCH, false>(tile, Q, kahan, grid, fgrid, a, f, s);
+    else if constexpr (!BATCH) launch_mode<DS_PHI, BATCH, false>(tile, Q, kahan, grid, fgrid, a, f, s);
 }
 
 SymShape direct_sym_shape(int sms, int64_t pairs) {
     SymShape sh;
     int occ = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, direct_sym_kernel<1, DS_ACC, false, DS_H, false>,
-                                                  DsShape<DS_H>::WARPS * 32, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, direct_sym_kernel<1, DS_ACC, false, DS_H, false, DS_T>,
+                                                  DsShape<DS_H, DS_T>::WARPS * 32, 0);
     sh.slots = (int64_t)sms * std::max(occ, 1);
-    sh.Q = direct_sym_slices(pairs, sh.slots, DsShape<DS_H>::QMAX);
+    sh.Q = direct_sym_slices(pairs, sh.slots, DsShape<DS_H, DS_T>::QMAX);
     return sh;
 }
 
@@ -472,24 +500,27 @@ int direct_sym_slices(int64_t pairs, int64_t slots, int qmax) {
 
 struct DsPlan {
     int64_t nt, NP, slots, max_pairs, need;  // need: float4s of scratch
-    int Q;
+    int tile, Q;
+    bool counted;               // CTAs take units from the counter (else one unit per CTA)
     std::vector<int64_t> rows;  // band b covers tile rows [rows[b], rows[b + 1])
 };
 
 static DsPlan ds_plan(const gb_direct *h, int64_t n) {
     DsPlan p;
-    p.nt = (n + DS_T - 1) / DS_T;
+    p.tile = n <= DS_SMALL_N && sym_one_band(n, DS_SMALL_T, DS_SMALL_Q, h->sym_band) ? DS_SMALL_T : DS_T;
+    p.nt = (n + p.tile - 1) / p.tile;
     p.NP = p.nt * (p.nt + 1) / 2;
     const SymShape sh = direct_sym_shape(h->sms, p.NP);
     p.slots = sh.slots;
-    p.Q = sh.Q;
+    p.Q = p.tile == DS_SMALL_T ? DS_SMALL_Q : sh.Q;
     // Tile pairs per band: the handle's slot budget (larger systems run in
     // bands of tile rows, so the scratch stays bounded at any N).
-    const int64_t budget = h->sym_band / ((int64_t)sizeof(float4) * DS_T * (p.Q + 1));
+    const int64_t budget = h->sym_band / ((int64_t)sizeof(float4) * p.tile * (p.Q + 1));
     p.max_pairs = sym_bands(p.nt, budget, p.rows);
+    p.counted = p.max_pairs * p.Q > p.slots;
     // Row slots, column slots, the running sums between bands, the counter.
     const int64_t aux = p.rows.size() > 2 ? 2 * n : 0;
-    p.need = p.max_pairs * p.Q * DS_T + p.max_pairs * DS_T + aux + 1;
+    p.need = p.max_pairs * p.Q * p.tile + p.max_pairs * p.tile + aux + 1;
     return p;
 }
 
@@ -510,8 +541,8 @@ int run_direct_sym(gb_direct *h, int mode, const float4 *xm, float4 *vel, float4
     a.vel = vel;
     a.acc = acc;
     a.rowpart = h->sym;
-    a.colpart = h->sym + pl.max_pairs * pl.Q * DS_T;
-    a.counter = (unsigned long long *)(h->sym + pl.need - 1);
+    a.colpart = h->sym + pl.max_pairs * pl.Q * pl.tile;
+    a.counter = pl.counted ? (unsigned long long *)(h->sym + pl.need - 1) : nullptr;
     a.n = n;
     a.nt = pl.nt;
     a.eps2 = eps2;
@@ -520,7 +551,7 @@ int run_direct_sym(gb_direct *h, int mode, const float4 *xm, float4 *vel, float4
     DsFix f{};
     f.rowpart = a.rowpart;
     f.colpart = a.colpart;
-    f.aux = a.colpart + pl.max_pairs * DS_T;
+    f.aux = a.colpart + pl.max_pairs * pl.tile;
     f.xm = const_cast<float4 *>(xm);
     f.vel = vel;
     f.acc = acc;
@@ -541,9 +572,9 @@ int run_direct_sym(gb_direct *h, int mode, const float4 *xm, float4 *vel, float4
         f.Ib = Ib;
         f.Ie = Ie;
         f.p0 = a.p0;
-        GB_CUDA_TRY(cudaMemsetAsync(a.counter, 0, sizeof(unsigned long long), s));
-        launch_pass<false>(mode, phi != nullptr && mode != DS_PHI, pl.Q, kahan,
-                           (unsigned)std::min(pl.slots, a.NU), (unsigned)((n - Ib * DS_T + 31) / 32), a, f, s);
+        if (pl.counted) GB_CUDA_TRY(cudaMemsetAsync(a.counter, 0, sizeof(unsigned long long), s));
+        launch_pass<false>(mode, phi != nullptr && mode != DS_PHI, pl.tile, pl.Q, kahan,
+                           (unsigned)std::min(pl.slots, a.NU), (unsigned)((n - Ib * pl.tile + 31) / 32), a, f, s);
         GB_CUDA_TRY(cudaGetLastError());
         h->launches += 2;
     }
@@ -586,7 +617,7 @@ int run_batch_sym(const SymBatch &b, int mode, const float4 *xm, float4 *vel, fl
     f.dt = dt;
     f.accumulate = (flags & GB_ACCUMULATE) ? 1 : 0;
     GB_CUDA_TRY(cudaMemsetAsync(a.counter, 0, sizeof(unsigned long long), s));
-    launch_pass<true>(mode, false, b.Q, !(flags & GB_PLAIN_FP32), (unsigned)b.P, (unsigned)b.nfb, a, f, s);
+    launch_pass<true>(mode, false, DS_T, b.Q, !(flags & GB_PLAIN_FP32), (unsigned)b.P, (unsigned)b.nfb, a, f, s);
     GB_CUDA_TRY(cudaGetLastError());
     return GB_OK;
 }
