@@ -362,7 +362,16 @@ __global__ void __launch_bounds__(SYM_WARPS * 32) adjoint_vjp_sym_kernel(SymArgs
 // d.w_source) stay in registers and are written negated.  On the diagonal
 // tile a pair (t, s) counts when t < s; the self pair is exactly zero.
 constexpr int SYM2_T = 512;
-constexpr int SYM2_WARPS = 4;
+template <int TILE>
+constexpr int SYM2_WARPS = TILE / 128;
+// Small systems (at most SYM2_SMALL_N particles): tiles of 256, two warps, four
+// source slices per tile pair.  As in the force pass the time is one unit's
+// length while the units fit one wave, and half of it here.  Microseconds per
+// VJP, tiles of 512 / 256: 1,000: 20.3 / 12.0; 4,096: 20.7 / 18.7; 6,144:
+// 47.8 / 32.4; 8,000: 60.9 / 53.6; beyond that the second wave's share falls
+// and the slots of the larger tiles are half as many.
+constexpr int SYM2_SMALL_T = 256, SYM2_SMALL_Q = 4;
+constexpr int64_t SYM2_SMALL_N = 8192;
 
 struct Sym2Args {
     const float4 *__restrict__ xm;
@@ -370,7 +379,7 @@ struct Sym2Args {
     const float4 *__restrict__ la;
     float4 *__restrict__ rowpart;  // NU x SYM2_T (one row slot per unit)
     float4 *__restrict__ colpart;  // band pairs x SYM2_T
-    unsigned long long *counter;   // zero at launch
+    unsigned long long *counter;   // zero at launch; NULL: one unit per CTA
     int64_t n, nt, NU, p0;         // units of the band, its first tile pair
     float eps2, h;
     int prime;
@@ -454,18 +463,21 @@ __device__ __forceinline__ void sym2_round(const float4 *__restrict__ sxm, const
     }
 }
 
-template <int Q>
-__global__ void __launch_bounds__(SYM2_WARPS * 32, 4) adjoint_vjp_sym2_kernel(Sym2Args a) {
-    constexpr int G = 16 / Q, SPAN = G * 32;
-    __shared__ float4 sxm[SYM2_T], sw[SYM2_T], sacc[SYM2_T];
+template <int Q, int TILE>
+__global__ void __launch_bounds__(SYM2_WARPS<TILE> * 32, 16 / SYM2_WARPS<TILE>) adjoint_vjp_sym2_kernel(Sym2Args a) {
+    constexpr int WARPS = SYM2_WARPS<TILE>, G = TILE / 32 / Q, SPAN = G * 32;
+    static_assert(G >= WARPS, "each warp of a round takes its own source group");
+    __shared__ float4 sxm[TILE], sw[TILE], sacc[TILE];
     __shared__ long long s_unit;
     __shared__ int s_gend, s_ntgt;  // source groups and targets of the unit that hold particles
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, tid = threadIdx.x;
     const int64_t NU = a.NU;
     const f2 EPS2 = pack2(a.eps2, a.eps2), NEG3 = pack2(-3.f, -3.f);
+    if (tid == 0) s_unit = -1;
     for (;;) {
         __syncthreads();  // the previous unit is done with s_unit and shared memory
-        if (tid == 0) s_unit = (long long)atomicAdd(a.counter, 1ull);
+        if (tid == 0)
+            s_unit = a.counter ? (long long)atomicAdd(a.counter, 1ull) : s_unit < 0 ? (long long)blockIdx.x : (long long)NU;
         __syncthreads();
         f2 TX[2], TY[2], TZ[2], TNM[2], TWX[2], TWY[2], TWZ[2], NX[2], NY[2], NZ[2], NG[2];
         bool diag;
@@ -485,15 +497,15 @@ __global__ void __launch_bounds__(SYM2_WARPS * 32, 4) adjoint_vjp_sym2_kernel(Sy
         // Padding of the last tile (zero mass and zero w) adds exact zeros:
         // its source groups and all-padding target warps are skipped.
         if (tid == 0) {
-            s_gend = (int)((min(a.n - J * SYM2_T, (int64_t)SYM2_T) + 31) / 32);
-            s_ntgt = (int)min(a.n - I * SYM2_T, (int64_t)SYM2_T);
+            s_gend = (int)((min(a.n - J * TILE, (int64_t)TILE) + 31) / 32);
+            s_ntgt = (int)min(a.n - I * TILE, (int64_t)TILE);
         }
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             float4 x[2], w[2];
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
-                const int64_t i = I * SYM2_T + 128 * wib + 32 * (2 * h + e) + lane;
+                const int64_t i = I * TILE + 128 * wib + 32 * (2 * h + e) + lane;
                 x[e] = i < a.n ? __ldg(a.xm + i) : make_float4(0.f, 0.f, 0.f, 0.f);
                 w[e] = sym2_w(a, i);
             }
@@ -507,9 +519,9 @@ __global__ void __launch_bounds__(SYM2_WARPS * 32, 4) adjoint_vjp_sym2_kernel(Sy
             NX[h] = NY[h] = NZ[h] = NG[h] = 0ull;
         }
         // Stage the slice's sources (tile-local indices sl*SPAN .. +SPAN-1).
-        for (int t = tid; t < SPAN; t += SYM2_WARPS * 32) {
+        for (int t = tid; t < SPAN; t += WARPS * 32) {
             const int tt = sl * SPAN + t;
-            const int64_t j = J * SYM2_T + tt;
+            const int64_t j = J * TILE + tt;
             sxm[tt] = j < a.n ? __ldg(a.xm + j) : make_float4(0.f, 0.f, 0.f, 0.f);
             sw[tt] = sym2_w(a, j);
             sacc[tt] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -517,7 +529,7 @@ __global__ void __launch_bounds__(SYM2_WARPS * 32, 4) adjoint_vjp_sym2_kernel(Sy
         }
         __syncthreads();
         for (int r = 0; r < G; ++r) {
-            const int g = gbase + (((G / 4) * wib + r) & (G - 1));
+            const int g = gbase + (((G / WARPS) * wib + r) & (G - 1));
             // Diagonal tile: targets 128 w .. 128 w + 127 against sources
             // 32 g .. 32 g + 31; no pair has t < s when 4 w > g.
             // Warp-uniform branches; every warp still reaches the barrier.
@@ -534,9 +546,9 @@ __global__ void __launch_bounds__(SYM2_WARPS * 32, 4) adjoint_vjp_sym2_kernel(Sy
         const int64_t u = s_unit;
         const int64_t p = u / Q;
         const int sl = (int)(u - p * Q);
-        for (int t = tid; t < SPAN; t += SYM2_WARPS * 32) {
+        for (int t = tid; t < SPAN; t += WARPS * 32) {
             const int tt = sl * SPAN + t;
-            a.colpart[p * SYM2_T + tt] = sacc[tt];
+            a.colpart[p * TILE + tt] = sacc[tt];
         }
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -545,7 +557,7 @@ __global__ void __launch_bounds__(SYM2_WARPS * 32, 4) adjoint_vjp_sym2_kernel(Sy
             unpack2(NY[h], y0, y1);
             unpack2(NZ[h], z0, z1);
             unpack2(NG[h], g0, g1);
-            float4 *row = a.rowpart + u * SYM2_T + 128 * wib + 64 * h + lane;
+            float4 *row = a.rowpart + u * TILE + 128 * wib + 64 * h + lane;
             row[0] = make_float4(-x0, -y0, -z0, -g0);
             row[32] = make_float4(-x1, -y1, -z1, -g1);
         }
@@ -571,29 +583,44 @@ struct Sym2Fix {
 // complete and gets the elementwise part of the backward step; one past the
 // band keeps its running sum in aux.  Later bands never read a finished
 // tile, so its adjoint state may change.  One band (Ib = 0, Ie = nt) is the
-// whole pass.
-__global__ void adjoint_sym2_fixup_kernel(Sym2Fix f) {
-    const int64_t i = f.Ib * SYM2_T + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= f.n) return;
-    const int64_t T = i / SYM2_T, r = i - T * SYM2_T;
+// whole pass.  A CTA takes 32 particles: warp w adds slots w, w + 8, ...
+// (512-byte rows), and warp 0 adds the warps' sums in order.  n = 65,536:
+// 38 us against 55 us with one thread for all slots of a particle, 4,096: 3.5
+// us against 4.8.
+constexpr int SYM2_FIX_WARPS = 8;
+
+template <int TILE>
+__global__ void __launch_bounds__(SYM2_FIX_WARPS * 32) adjoint_sym2_fixup_kernel(Sym2Fix f) {
+    __shared__ float4 part[SYM2_FIX_WARPS][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t i0 = f.Ib * TILE + (int64_t)blockIdx.x * 32, i = i0 + lane;
+    const int64_t T = i0 / TILE, r = i - T * TILE;
     const bool in_band = T < f.Ie;
+    const int64_t R = in_band ? (f.nt - T) * f.Q : 0;          // row slots
+    const int64_t C = (in_band ? T : f.Ie - 1) - f.Ib + 1;     // column slots
+    const int64_t rbase = (sym_base(T, f.nt) - f.p0) * f.Q;
     float gx = 0.f, gy = 0.f, gz = 0.f, gm = 0.f;
-    if (f.Ib > 0) {
-        const float4 v = f.aux[i];
-        gx = v.x; gy = v.y; gz = v.z; gm = v.w;
-    }
-    if (in_band) {
-        const int64_t u0 = (sym_base(T, f.nt) - f.p0) * f.Q, u1 = u0 + (f.nt - T) * f.Q;
-        for (int64_t u = u0; u < u1; ++u) {
-            const float4 v = f.rowpart[u * SYM2_T + r];
-            gx += v.x; gy += v.y; gz += v.z; gm += v.w;
-        }
-    }
-    const int64_t last = in_band ? T : f.Ie - 1;
-    for (int64_t I2 = f.Ib; I2 <= last; ++I2) {
-        const float4 v = f.colpart[(sym_base(I2, f.nt) + (T - I2) - f.p0) * SYM2_T + r];
+    auto add = [&](float4 v) {
         gx += v.x; gy += v.y; gz += v.z; gm += v.w;
+    };
+    // Slots of padded particles (i >= n) lie inside the scratch; their sums are dropped below.
+    const float4 *row = f.rowpart + rbase * TILE + r;
+    const int nr = (int)R, nc = (int)C;
+#pragma unroll 4
+    for (int k = w; k < nr; k += SYM2_FIX_WARPS) add(row[(int64_t)k * TILE]);
+    const float4 *col = f.colpart + (T - f.p0) * TILE + r;
+#pragma unroll 4
+    for (int k = (nr + SYM2_FIX_WARPS - 1 - w) / SYM2_FIX_WARPS * SYM2_FIX_WARPS + w - nr; k < nc; k += SYM2_FIX_WARPS) {
+        const int64_t I2 = f.Ib + k;
+        add(col[(sym_base(I2, f.nt) - I2) * TILE]);
     }
+    part[w][lane] = make_float4(gx, gy, gz, gm);
+    __syncthreads();
+    if (w != 0 || i >= f.n) return;
+    gx = gy = gz = gm = 0.f;
+    if (f.Ib > 0) add(f.aux[i]);
+#pragma unroll
+    for (int q = 0; q < SYM2_FIX_WARPS; ++q) add(part[q][lane]);
     if (!in_band) {
         f.aux[i] = make_float4(gx, gy, gz, gm);
         return;
@@ -676,18 +703,27 @@ extern "C" int gb_adjoint_step(gb_direct_t *h, const float *xm, float *lx, float
     if (!(eps2 > 0.f)) return fail(GB_EINVAL, "eps2 must be > 0");
     cudaStream_t s = (cudaStream_t)stream;
     if (h->adj_variant == 2) {
-        const int64_t nt = (n + SYM2_T - 1) / SYM2_T, NP = nt * (nt + 1) / 2;
+        // Small tiles where one band holds their slots.
+        const bool small = n <= SYM2_SMALL_N && sym_one_band(n, SYM2_SMALL_T, SYM2_SMALL_Q, h->sym_band);
+        const int tile = small ? SYM2_SMALL_T : SYM2_T;
+        const int64_t nt = (n + tile - 1) / tile, NP = nt * (nt + 1) / 2;
         int occs = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occs, adjoint_vjp_sym2_kernel<1>, SYM2_WARPS * 32, 0);
+        if (small)
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occs, adjoint_vjp_sym2_kernel<SYM2_SMALL_Q, SYM2_SMALL_T>,
+                                                          SYM2_WARPS<SYM2_SMALL_T> * 32, 0);
+        else
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occs, adjoint_vjp_sym2_kernel<1, SYM2_T>,
+                                                          SYM2_WARPS<SYM2_T> * 32, 0);
         const int64_t slots = (int64_t)h->sms * std::max(occs, 1);
-        const int Q = direct_sym_slices(NP, slots, 16 / SYM2_WARPS);
+        const int Q = small ? SYM2_SMALL_Q : direct_sym_slices(NP, slots, 16 / SYM2_WARPS<SYM2_T>);
         // Bands of tile rows within the handle's slot budget, as for the
         // symmetric force pass.
         std::vector<int64_t> rows;
         const int64_t max_pairs =
-            sym_bands(nt, h->sym_band / ((int64_t)sizeof(float4) * SYM2_T * (Q + 1)), rows);
+            sym_bands(nt, h->sym_band / ((int64_t)sizeof(float4) * tile * (Q + 1)), rows);
         const int64_t aux = rows.size() > 2 ? n : 0;
-        const int64_t need = max_pairs * Q * SYM2_T + max_pairs * SYM2_T + aux + 1;  // + the unit counter
+        const int64_t need = max_pairs * Q * tile + max_pairs * tile + aux + 1;  // + the unit counter
+        const bool counted = max_pairs * Q > slots;
         if (need * (int64_t)sizeof(float4) <= SYM_MAX_BYTES) {
             GB_TRY(ensure_sym(h, need));
             Sym2Args a;
@@ -695,8 +731,8 @@ extern "C" int gb_adjoint_step(gb_direct_t *h, const float *xm, float *lx, float
             a.lv = (const float4 *)lv;
             a.la = (const float4 *)la;
             a.rowpart = h->sym;
-            a.colpart = h->sym + max_pairs * Q * SYM2_T;
-            a.counter = (unsigned long long *)(h->sym + need - 1);
+            a.colpart = h->sym + max_pairs * Q * tile;
+            a.counter = counted ? (unsigned long long *)(h->sym + need - 1) : nullptr;
             a.n = n;
             a.nt = nt;
             a.eps2 = eps2;
@@ -705,7 +741,7 @@ extern "C" int gb_adjoint_step(gb_direct_t *h, const float *xm, float *lx, float
             Sym2Fix f;
             f.rowpart = a.rowpart;
             f.colpart = a.colpart;
-            f.aux = a.colpart + max_pairs * SYM2_T;
+            f.aux = a.colpart + max_pairs * tile;
             f.lx = (float4 *)lx;
             f.lv = (float4 *)lv;
             f.la = (float4 *)la;
@@ -724,12 +760,17 @@ extern "C" int gb_adjoint_step(gb_direct_t *h, const float *xm, float *lx, float
                 f.Ie = rows[b + 1];
                 f.p0 = a.p0;
                 const unsigned P = (unsigned)std::min(slots, a.NU);
-                GB_CUDA_TRY(cudaMemsetAsync(a.counter, 0, sizeof(unsigned long long), s));
-                if (Q == 1) adjoint_vjp_sym2_kernel<1><<<P, SYM2_WARPS * 32, 0, s>>>(a);
-                else if (Q == 2) adjoint_vjp_sym2_kernel<2><<<P, SYM2_WARPS * 32, 0, s>>>(a);
-                else adjoint_vjp_sym2_kernel<4><<<P, SYM2_WARPS * 32, 0, s>>>(a);
+                if (counted) GB_CUDA_TRY(cudaMemsetAsync(a.counter, 0, sizeof(unsigned long long), s));
+                const unsigned b1 = SYM2_WARPS<SYM2_T> * 32;
+                if (small)
+                    adjoint_vjp_sym2_kernel<SYM2_SMALL_Q, SYM2_SMALL_T><<<P, SYM2_WARPS<SYM2_SMALL_T> * 32, 0, s>>>(a);
+                else if (Q == 1) adjoint_vjp_sym2_kernel<1, SYM2_T><<<P, b1, 0, s>>>(a);
+                else if (Q == 2) adjoint_vjp_sym2_kernel<2, SYM2_T><<<P, b1, 0, s>>>(a);
+                else adjoint_vjp_sym2_kernel<4, SYM2_T><<<P, b1, 0, s>>>(a);
                 GB_CUDA_TRY(cudaGetLastError());
-                adjoint_sym2_fixup_kernel<<<(unsigned)((n - f.Ib * SYM2_T + 255) / 256), 256, 0, s>>>(f);
+                const unsigned fgrid = (unsigned)((n - f.Ib * tile + 31) / 32);
+                if (small) adjoint_sym2_fixup_kernel<SYM2_SMALL_T><<<fgrid, SYM2_FIX_WARPS * 32, 0, s>>>(f);
+                else adjoint_sym2_fixup_kernel<SYM2_T><<<fgrid, SYM2_FIX_WARPS * 32, 0, s>>>(f);
                 GB_CUDA_TRY(cudaGetLastError());
                 h->launches += 2;
             }
