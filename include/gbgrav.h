@@ -385,6 +385,18 @@ int gb_adjoint_step(gb_direct_t *h, const float *xm, float *lx, float *lv,
                     float *la, float *lm, int64_t n, float G, float eps2,
                     float dt, int prime, void *stream);
 
+/* nsteps KDK steps of gb_direct_kdk in place; traj row k (n float4 records)
+ * gets xm after step k + 1. */
+int gb_adjoint_trajectory(gb_direct_t *h, float *xm, float *vel, float *acc,
+                          float *traj, int64_t n, float G, float eps2,
+                          float dt, int64_t nsteps, int flags, void *stream);
+/* gb_adjoint_step (prime 0) over nsteps steps in reverse.  traj row k holds
+ * the positions after step k + 1 for k < nsteps - 1 (NULL for one step),
+ * x_end those after the last. */
+int gb_adjoint_segment(gb_direct_t *h, const float *traj, const float *x_end,
+                       float *lx, float *lv, float *la, float *lm, int64_t n,
+                       float G, float eps2, float dt, int64_t nsteps,
+                       void *stream);
 /* Pair evaluation of the adjoint:
  *   2 (default) every unordered pair once, applied to both particles, in
  *     packed FP32x2 arithmetic with CTAs taking tile-pair units from a

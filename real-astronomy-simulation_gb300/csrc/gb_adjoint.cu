@@ -868,6 +868,37 @@ extern "C" int gb_adjoint_step(gb_direct_t *h, const float *xm, float *lx, float
     return GB_OK;
 }
 
+extern "C" int gb_adjoint_trajectory(gb_direct_t *h, float *xm, float *vel, float *acc, float *traj, int64_t n, float G,
+                                     float eps2, float dt, int64_t nsteps, int flags, void *stream) {
+    if (!h) return fail(GB_EINVAL, "handle is NULL");
+    if (n < 0 || n > h->n_max) return fail(GB_EINVAL, "n=%lld outside [0, n_max=%lld]", (long long)n,
+                                           (long long)h->n_max);
+    if (nsteps < 0) return fail(GB_EINVAL, "nsteps < 0");
+    if (flags & ~GB_PLAIN_FP32) return fail(GB_EINVAL, "flags 0x%x: only GB_PLAIN_FP32 applies", flags);
+    if (n > 0 && nsteps > 0) {
+        if (!traj) return fail(GB_EINVAL, "traj is NULL");
+        if (!aligned16(traj)) return fail(GB_EINVAL, "traj is not 16-byte aligned");
+    }
+    for (int64_t k = 0; k < nsteps; ++k) {
+        GB_TRY(gb_direct_kdk(h, xm, vel, acc, n, G, eps2, dt, 1, flags, stream));
+        if (n > 0)
+            GB_CUDA_TRY(cudaMemcpyAsync(traj + 4 * k * n, xm, (size_t)n * 4 * sizeof(float), cudaMemcpyDeviceToDevice,
+                                        (cudaStream_t)stream));
+    }
+    return GB_OK;
+}
+
+extern "C" int gb_adjoint_segment(gb_direct_t *h, const float *traj, const float *x_end, float *lx, float *lv,
+                                  float *la, float *lm, int64_t n, float G, float eps2, float dt, int64_t nsteps,
+                                  void *stream) {
+    if (nsteps < 0) return fail(GB_EINVAL, "nsteps < 0");
+    if (n > 0 && nsteps > 1 && !traj) return fail(GB_EINVAL, "traj is NULL");
+    for (int64_t k = nsteps - 1; k >= 0; --k)
+        GB_TRY(gb_adjoint_step(h, k == nsteps - 1 ? x_end : traj + 4 * k * n, lx, lv, la, lm, n, G, eps2, dt, 0,
+                               stream));
+    return GB_OK;
+}
+
 extern "C" int gb_adjoint_set_variant(gb_direct_t *h, int variant) {
     if (!h) return fail(GB_EINVAL, "handle is NULL");
     if (variant < 0 || variant > 2) return fail(GB_EINVAL, "variant must be 0, 1 or 2 (got %d)", variant);
