@@ -367,7 +367,7 @@ constexpr int SYM2_WARPS = TILE / 128;
 // Small systems (at most SYM2_SMALL_N particles): tiles of 256, two warps, four
 // source slices per tile pair.  As in the force pass the time is one unit's
 // length while the units fit one wave, and half of it here.  Microseconds per
-// VJP, tiles of 512 / 256: 1,000: 20.3 / 12.0; 4,096: 20.7 / 18.7; 6,144:
+// VJP, tiles of 512 / 256: 1,000: 20.3 / 10.2; 4,096: 20.7 / 18.7; 6,144:
 // 47.8 / 32.4; 8,000: 60.9 / 53.6; beyond that the second wave's share falls
 // and the slots of the larger tiles are half as many.
 constexpr int SYM2_SMALL_T = 256, SYM2_SMALL_Q = 4;
@@ -406,10 +406,16 @@ __device__ __forceinline__ void sym2_round(const float4 *__restrict__ sxm, const
     // 3 m_t for the lane's targets: d.u = m_s d.w_t - m_t d.w_s, so
     // -3 d.u = (-3 m_s) d.w_t + (3 m_t) d.w_s from the two dot products.
     const f2 TM3[2] = {mul2(TNM[0], NEG3), mul2(TNM[1], NEG3)};
+    // The next step's source is read one step ahead: where a block is alone on
+    // its SM the read's latency was not covered (VJP and fix-up of 1,000
+    // particles: 18.7 to 16.7 us; of 4,096 and more: the same).
+    float4 xn = sxm[g * 32 + lane], wn = sw[g * 32 + lane];
 #pragma unroll 2
     for (int k = 0; k < 32; ++k) {
-        const int jj = g * 32 + ((lane + k) & 31);
-        const float4 xs = sxm[jj], ws = sw[jj];
+        const int jj = g * 32 + ((lane + k) & 31), jn = g * 32 + ((lane + k + 1) & 31);
+        const float4 xs = xn, ws = wn;
+        xn = sxm[jn];
+        wn = sw[jn];
         const f2 sx = pack2(xs.x, xs.x), sy = pack2(xs.y, xs.y), sz = pack2(xs.z, xs.z);
         const f2 sm = pack2(xs.w, xs.w);
         const f2 sm3 = mul2(sm, NEG3);

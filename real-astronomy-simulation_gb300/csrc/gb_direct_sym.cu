@@ -46,7 +46,7 @@ constexpr int DS_ACC = 0, DS_KDK = 1, DS_PHI = 2;
 // per tile pair its units stay short enough for small systems too.
 template <int H, int T>
 struct DsShape {
-    static constexpr int WT = 64 * H, WARPS = T / WT, MIN_CTAS = H == 4 ? 8 : 12;
+    static constexpr int WT = 64 * H, WARPS = T / WT, MIN_CTAS = 8;
     static constexpr int QMAX = T / 32 / WARPS;  // each warp of a round takes its own source group
     static_assert(WARPS * WT == T, "a CTA's warps cover one tile");
 };
@@ -58,7 +58,7 @@ constexpr int DS_H = 4;
 // (300 tile pairs, 1,200 units) the small units still run in one wave, so each
 // CTA takes the unit of its index and the counter with its memset is left out.
 // Microseconds per KDK step, tiles of 512 with the counter / 512 without / 256:
-// 1,000: 18.5 / 14.7 / 11.6; 4,096: 18.5 / 15.7 / 14.6; 6,144: - / 26.2 / 21.1;
+// 1,000: 18.5 / 14.7 / 10.6; 4,096: 18.5 / 15.7 / 12.9; 6,144: - / 26.2 / 19.8;
 // past the wave the twice as many slots cost more: 8,000: - / 32.9 / 37.2.
 constexpr int DS_SMALL_T = 256, DS_SMALL_H = 2, DS_SMALL_Q = 4;
 constexpr int64_t DS_SMALL_N = 6144;
@@ -100,10 +100,16 @@ __device__ __forceinline__ void ds_round(const float4 *__restrict__ sxm, float4 
                                          f2 EPS2, const f2 (&TX)[H], const f2 (&TY)[H], const f2 (&TZ)[H],
                                          const f2 (&TM)[H], f2 (&NX)[H], f2 (&NY)[H], f2 (&NZ)[H],
                                          f2 (&NW)[H]) {
+    // Small tiles read the next step's source one step ahead: with few warps
+    // on an SM the read's latency was not covered (force kernel at 1,000:
+    // 8.1 to 6.3 us, 4,096: 10.2 to 9.4, 6,144: 16.9 to 15.8).  The large shape
+    // has 16 warps an SM for that and no registers left.
+    float4 xn = sxm[g * 32 + lane];
 #pragma unroll DS_K_UNROLL
     for (int k = 0; k < 32; ++k) {
         const int jj = g * 32 + ((lane + k) & 31);
-        const float4 xs = sxm[jj];
+        const float4 xs = H == DS_SMALL_H ? xn : sxm[jj];
+        if (H == DS_SMALL_H) xn = sxm[g * 32 + ((lane + k + 1) & 31)];
         const f2 sx = pack2(xs.x, xs.x), sy = pack2(xs.y, xs.y), sz = pack2(xs.z, xs.z);
         const f2 sm = pack2(xs.w, xs.w);
         f2 PX = 0ull, PY = 0ull, PZ = 0ull, PW = 0ull;
