@@ -1296,14 +1296,16 @@ extern "C" int gb_bh_energy(gb_bh_t *h, const float *xm, const float *vel, const
 }
 
 // One CTA runs the radix sort's look-back for tile 1 of a two-tile status
-// array.  publish_first = 1: each thread first publishes tile 0's prefix
-// (its digit d as the count), so the look-back returns d; 0: tile 0 never
+// array.  publish_first = 1: each thread first publishes tile 0's count
+// (its digit d), so the look-back returns d; 0: tile 0 never
 // publishes and every wait runs out after spin_limit polls.
 __global__ void sort_wait_probe_kernel(uint32_t *status, int spin_limit, int publish_first, uint32_t *excl,
                                        unsigned long long *diag) {
     const int d = threadIdx.x;
-    if (publish_first) st_relaxed_gpu(status + d, RS_PRE | (uint32_t)d);
-    excl[d] = rs_lookback(status, 1, d, 1u, spin_limit, diag);
+    if (publish_first) st_relaxed_gpu(status + d, RS_AGG | (uint32_t)d);
+    const RsStatus st(status, 2);
+    rs_publish(st, 1, d, 1u);
+    excl[d] = rs_lookback(st, 1, d, 1u, spin_limit, diag);
 }
 
 extern "C" int gb_sort_wait_probe(int spin_limit, int publish_first, uint32_t *excl_out, uint64_t *timeouts_out) {
@@ -1313,12 +1315,12 @@ extern "C" int gb_sort_wait_probe(int spin_limit, int publish_first, uint32_t *e
     uint32_t *status = nullptr, *excl = nullptr;
     unsigned long long *diag = nullptr;
     int rc = GB_OK;
-    if (cudaMalloc(&status, sizeof(uint32_t) * 2 * RS_BINS) != cudaSuccess ||
+    if (cudaMalloc(&status, sizeof(uint32_t) * radix_status_words(2 * RS_TILE)) != cudaSuccess ||
         cudaMalloc(&excl, sizeof(uint32_t) * RS_BINS) != cudaSuccess ||
         cudaMalloc(&diag, sizeof(unsigned long long) * DIAG_COUNT) != cudaSuccess) {
         rc = fail(GB_ENOMEM, "gb_sort_wait_probe: device allocation failed");
     }
-    if (rc == GB_OK && (cudaMemset(status, 0, sizeof(uint32_t) * 2 * RS_BINS) != cudaSuccess ||
+    if (rc == GB_OK && (cudaMemset(status, 0, sizeof(uint32_t) * radix_status_words(2 * RS_TILE)) != cudaSuccess ||
                         cudaMemset(diag, 0, sizeof(unsigned long long) * DIAG_COUNT) != cudaSuccess))
         rc = fail(GB_ECUDA, "gb_sort_wait_probe: memset failed");
     if (rc == GB_OK) {
