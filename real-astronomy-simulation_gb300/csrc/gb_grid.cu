@@ -101,7 +101,7 @@ __device__ __forceinline__ GridPart cta_merge(GridPart p, GridPart *w) {
 
 // Bound by the latency of its tail, the merge and the FP64 divisions of the
 // geometry.  The last CTA's threads share the merge of the block partials: at
-// n = 1,000,000 11.6 us, against 66.9 us with 608 partials read one after the
+// n = 1,000,000 10.8 us, against 71 us with 608 partials read one after the
 // other by one thread.
 __global__ void __launch_bounds__(GRID_THREADS)
 grid_reduce_kernel(const float4 *__restrict__ xm, const float *__restrict__ hsml, const int *__restrict__ is_star,
@@ -111,16 +111,33 @@ grid_reduce_kernel(const float4 *__restrict__ xm, const float *__restrict__ hsml
     float mn0 = INFINITY, mn1 = INFINITY, mn2 = INFINITY, mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY;
     float hm = -INFINITY;
     unsigned long long cnt = 0, bad = 0;
-    for (int64_t i = (int64_t)blockIdx.x * GRID_THREADS + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * GRID_THREADS) {
-        if (is_star && __ldg(is_star + i) != 0) continue;
-        const float4 p = __ldg(xm + i);
-        const float hv = __ldg(hsml + i);
-        if (!(isfinite(p.x) && isfinite(p.y) && isfinite(p.z) && isfinite(hv))) ++bad;
-        mn0 = fminf(mn0, p.x); mn1 = fminf(mn1, p.y); mn2 = fminf(mn2, p.z);
-        mx0 = fmaxf(mx0, p.x); mx1 = fmaxf(mx1, p.y); mx2 = fmaxf(mx2, p.z);
-        hm = fmaxf(hm, hv);
-        ++cnt;
+    // Four particles' loads at once: with one at a time, and its position read
+    // after its star flag, the kernel took 15.5 us at n = 1,000,000, now 10.8.
+    constexpr int U = 4;
+    const int64_t step = (int64_t)gridDim.x * GRID_THREADS;
+    for (int64_t i0 = (int64_t)blockIdx.x * GRID_THREADS + threadIdx.x; i0 < n; i0 += U * step) {
+        float4 p[U];
+        float hv[U];
+        int star[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int64_t i = i0 + u * step;
+            star[u] = 1;
+            if (i < n) {
+                star[u] = is_star ? __ldg(is_star + i) : 0;
+                p[u] = __ldg(xm + i);
+                hv[u] = __ldg(hsml + i);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (star[u] != 0) continue;
+            if (!(isfinite(p[u].x) && isfinite(p[u].y) && isfinite(p[u].z) && isfinite(hv[u]))) ++bad;
+            mn0 = fminf(mn0, p[u].x); mn1 = fminf(mn1, p[u].y); mn2 = fminf(mn2, p[u].z);
+            mx0 = fmaxf(mx0, p[u].x); mx1 = fmaxf(mx1, p[u].y); mx2 = fmaxf(mx2, p[u].z);
+            hm = fmaxf(hm, hv[u]);
+            ++cnt;
+        }
     }
     __shared__ GridPart wpart[GRID_THREADS / 32];
     __shared__ bool last;
