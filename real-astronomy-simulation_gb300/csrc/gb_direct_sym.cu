@@ -507,9 +507,14 @@ SymShape direct_sym_shape(int sms, int64_t pairs) {
 
 int direct_sym_slices(int64_t pairs, int64_t slots, int qmax) {
     // Source slices per tile pair: enough units that the last ones are a
-    // small share of each CTA's work.
+    // small share of each CTA's work.  Two slices pay below 16 units per slot,
+    // more only below 8: each slice adds a row slot for the fix-up to read.
+    // KDK steps, us, with 16 for all / this rule: 40,000: 518 / 487; 50,000:
+    // 800 / 757; 65,536: 1,290 / 1,257; 100 systems of 100 to 12,000: 465 / 447;
+    // up to 35,000 and from 80,000 the slices are the same.  With 8 for all:
+    // 90,000: 2,334 / 2,376.
     int Q = 1;
-    while (Q < qmax && pairs * Q < 16 * slots) Q *= 2;
+    while (Q < qmax && pairs * Q < (Q == 1 ? 16 : 8) * slots) Q *= 2;
     return Q;
 }
 

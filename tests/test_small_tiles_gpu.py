@@ -60,6 +60,23 @@ def test_direct_small_tiles_match_oracle(cuda_dev, orc, n):
     assert _rel(out[1], out[0]).max() < TOL
 
 
+@pytest.mark.parametrize("n", [36001, 50001, 65536])
+def test_direct_slices_match_oracle(cuda_dev, orc, n):
+    """8, 4 and 2 source slices per tile pair of 512."""
+    grav = importlib.import_module(PKG_NAME + ".solvers.gravity")
+    ic = importlib.import_module(PKG_NAME + ".ic")
+    pos, _, mass = (_f32(a) for a in ic.plummer(n, seed=n))
+    xm = torch.tensor(np.column_stack((pos, mass)), dtype=torch.float32, device=cuda_dev)
+    s = grav.DirectGravity(n, cuda_dev)
+    s.set_variant(2)
+    acc = torch.full_like(xm, 7.0)
+    s.acc(xm, acc, 1.0, 1e-4)
+    targets = np.random.default_rng(n).choice(n, 1024, replace=False)
+    ref = orc.direct_acc(pos, mass, 1.0, 1e-4, targets)
+    assert _rel(acc[:, :3].double().cpu().numpy()[targets], ref).max() < TOL
+    s.close()
+
+
 @pytest.mark.parametrize("prime", [0, 1])
 @pytest.mark.parametrize("n", [1, 255, 256, 257, 8191, 8192, 8193])
 def test_adjoint_small_tiles_match_large_tiles(cuda_dev, n, prime):
