@@ -4,8 +4,8 @@ Headline workload (one JSON line on rank 0): LBVH Barnes-Hut KDK steps on a
 1,000,000-particle exponential stellar disk (M = 5e10 Msun, Rd = 3 kpc,
 sech^2 z0 = 0.3 kpc, 10% dispersion, seed 0, galactic units), theta = 0.5,
 eps = 0.05 kpc, 30-bit Morton keys, dt = 1e-4.  A step is one full KDK step:
-fused kick+drift, bounding box, keys, radix sort, Karras build, bottom-up
-summaries, traversal with the closing kick.  Metric: particle-steps/s.
+fused kick+drift, bounding box, keys, radix sort, tree with its summaries,
+traversal with the closing kick.  Metric: particle-steps/s.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl gb|reference]
 
@@ -279,7 +279,7 @@ def bench_bh(args, dev, rank, world, dist):
                 if k in ("warp_node_reads", "warp_root_reads", "lane_interactions", "lane_tests")}
     del tmp
     # Roofline of the dominant kernel (traversal): algorithmic bytes per launch
-    # = node records read per warp (48 B two-children record per expansion,
+    # = node records read per group (48 B two-children record per expansion,
     # 32 B root record) + per particle: own leaf 16 B, order 4 B, velocity
     # 16 B read + 16 B write, acceleration 16 B write.
     trav_ms = res["stages_ms_per_step"]["traverse"]
@@ -288,33 +288,34 @@ def bench_bh(args, dev, rank, world, dist):
                     + BH_N * (16 + 4 + 16 + 16 + 16 + (4 if args.bh_traversal == 3 else 0)))
     hbm, src = _peaks()
     achieved = bytes_launch / (trav_ms / 1e3) / 1e9
-    res["roofline"] = {"kernel": "bh_traverse_kernel", "bound": "hbm", "achieved": achieved,
+    res["roofline"] = {"kernel": "bh_group_kernel" if args.bh_traversal == 3 else "bh_walk_kernel",
+                       "bound": "hbm", "achieved": achieved,
                        "peak": hbm, "peak_source": f"{src} (MEASURED_PEAKS.json hbm_gbs)"
                        if src == "measured" else "fallback 6800 GB/s",
                        "unit": "GB/s", "frac": achieved / hbm, "traffic": None,
                        "algorithmic_bytes_per_launch": bytes_launch,
                        "launch_ms": trav_ms}
-    traffic = _profiled_traffic("bh_traverse_1M_disk.md")
-    if traffic is not None and not _profile_current("bh_traverse_1M_disk.md", "gb_bh_traverse.cuh"):
+    traffic = _profiled_traffic("bh_walk_1M_disk.md")
+    if traffic is not None and not _profile_current("bh_walk_1M_disk.md", "gb_bh_traverse.cuh"):
         # The capture measured another revision of the kernel source: its
         # figures are not this kernel's.
-        res["roofline"]["traffic_source"] = ("none: profiles/bh_traverse_1M_disk.md was captured on "
+        res["roofline"]["traffic_source"] = ("none: profiles/bh_walk_1M_disk.md was captured on "
                                              "another revision of csrc/gb_bh_traverse.cuh")
         traffic = None
     if traffic is not None and BH_N == 1_000_000 and BH_BITS == 10:
         res["roofline"]["traffic"] = traffic
         res["roofline"]["traffic_source"] = ("ncu dram bytes of one launch on this workload "
-                                             "(profiles/bh_traverse_1M_disk.md)")
+                                             "(profiles/bh_walk_1M_disk.md)")
         # The kernel's actual limit is instruction issue, not HBM: the same
         # capture's issue-slot and pipe utilisation.
         res["roofline"]["observed_limit"] = {
-            "issue_active_pct": _profiled_metric("bh_traverse_1M_disk.md",
+            "issue_active_pct": _profiled_metric("bh_walk_1M_disk.md",
                                                  "smsp__issue_active.avg.pct_of_peak_sustained_active"),
-            "alu_pipe_pct": _profiled_metric("bh_traverse_1M_disk.md",
+            "alu_pipe_pct": _profiled_metric("bh_walk_1M_disk.md",
                                              "sm__pipe_alu_cycles_active.avg.pct_of_peak_sustained_active"),
-            "fma_pipe_pct": _profiled_metric("bh_traverse_1M_disk.md",
+            "fma_pipe_pct": _profiled_metric("bh_walk_1M_disk.md",
                                              "sm__pipe_fma_cycles_active.avg.pct_of_peak_sustained_active"),
-            "source": "ncu --set full capture of one launch (profiles/bh_traverse_1M_disk.md)"}
+            "source": "ncu --set full capture of one launch (profiles/bh_walk_1M_disk.md)"}
     # The same launch seen as FP32 work: 20 flop per monopole term, 10 per
     # acceptance test.
     flops = 20 * per_step["lane_interactions"] + 10 * per_step["lane_tests"]

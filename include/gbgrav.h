@@ -78,7 +78,8 @@ int gb_direct_set_tiles(gb_direct_t *h, int k, int warps, int ctas_per_sm);
 /* Inner-loop form: 0 = scalar FP32 (default), 1 = packed .f32x2 FP32, one
  * pass per target; 2 = symmetric packed .f32x2, each unordered pair once,
  * applied to both particles.  The symmetric pass keeps 8 KB slots per
- * 512 x 512 tile pair (N^2/32 bytes in all at large N); above the band
+ * 512 x 512 tile pair (N^2/32 bytes in all at large N; 4 KB per 256 x 256 up
+ * to 6,144 particles); above the band
  * budget (gb_direct_set_sym_band, 1 GiB by default) it runs in bands of tile
  * rows, two kernels per band, plus 32 bytes per particle of running sums.
  * Same results up to FP32 rounding order.  gb_direct_phi (and gb_energy)
@@ -199,7 +200,7 @@ int gb_bh_destroy(gb_bh_t *h);
 
 /* Device build: bounding box, Morton keys (bit-identical to morton_codes,
  * core/solvers/barnes_hut.py:27-46), stable radix sort (the permutation of
- * np.argsort(kind="stable"), :247), Karras tree (_build_radix, :84-121),
+ * np.argsort(kind="stable"), :247), binary radix tree (_build_radix, :84-121),
  * node summaries (_leaf_init/_accumulate/_finalize, :124-177). */
 int gb_bh_build(gb_bh_t *h, const float *xm, int64_t n, void *stream);
 
@@ -400,7 +401,8 @@ int gb_adjoint_segment(gb_direct_t *h, const float *traj, const float *x_end,
 /* Pair evaluation of the adjoint:
  *   2 (default) every unordered pair once, applied to both particles, in
  *     packed FP32x2 arithmetic with CTAs taking tile-pair units from a
- *     counter (8 KB slots per 512 x 512 tile pair, allocated on first use;
+ *     counter (8 KB slots per 512 x 512 tile pair, or 4 KB per 256 x 256 up
+ *     to 8,192 particles, allocated on first use;
  *     above the handle's band budget, gb_direct_set_sym_band, it runs in
  *     bands of tile rows with 16 bytes per particle of running sums);
  *   1 every unordered pair once, scalar FP32, static runs per CTA (scratch

@@ -2,7 +2,7 @@
 
 Mirrors ``BarnesHut(n, theta, softening, max_stack).compute(pos, mass, acc)``
 (core/solvers/barnes_hut.py:220-259).  Every stage (Morton keys, stable
-sort, Karras build, node summaries, traversal) runs on the device; keys,
+sort, tree with its summaries, traversal) runs on the device; keys,
 order and topology are bit-identical to the reference's and each particle
 accepts the same node set.  Extra keyword arguments: ``key_bits`` (21 = the
 reference's 63-bit keys, 10 = 30-bit keys), ``G`` (the reference compiles
