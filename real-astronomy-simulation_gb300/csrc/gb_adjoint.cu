@@ -897,6 +897,7 @@ extern "C" int gb_adjoint_trajectory(gb_direct_t *h, float *xm, float *vel, floa
 extern "C" int gb_adjoint_segment(gb_direct_t *h, const float *traj, const float *x_end, float *lx, float *lv,
                                   float *la, float *lm, int64_t n, float G, float eps2, float dt, int64_t nsteps,
                                   void *stream) {
+    if (!h) return fail(GB_EINVAL, "handle is NULL");
     if (nsteps < 0) return fail(GB_EINVAL, "nsteps < 0");
     if (n > 0 && nsteps > 1 && !traj) return fail(GB_EINVAL, "traj is NULL");
     for (int64_t k = nsteps - 1; k >= 0; --k)
