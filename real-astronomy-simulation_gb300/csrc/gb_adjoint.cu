@@ -393,67 +393,75 @@ __device__ __forceinline__ float4 sym2_w(const Sym2Args &a, int64_t i) {
     return make_float4(__fmaf_rn(a.h, lv.x, la.x), __fmaf_rn(a.h, lv.y, la.y), __fmaf_rn(a.h, lv.z, la.z), 0.f);
 }
 
+// A lane's four targets, two by two, with their sums.
+struct Sym2Half {
+    f2 TX, TY, TZ, TNM, TWX, TWY, TWZ, NX, NY, NZ, NG;
+};
+
+// One source against two of the lane's targets, HH the first (0) or the second
+// half; the source's sums in PX .. PG.  -3 d.u, with u = m_s w_t - m_t w_s, comes
+// from the two dot products: (-3 m_s) d.w_t + (3 m_t) d.w_s.  DIAG masks the
+// pairs with target index >= source index (diagonal tile).
+template <bool DIAG, int HH>
+__device__ __forceinline__ void sym2_half(Sym2Half &t, float4 xs, float4 ws, int jj, int lane, int wib, float eps2,
+                                          f2 &PX, f2 &PY, f2 &PZ, f2 &PG) {
+    const f2 sx = pack2(xs.x, xs.x), sy = pack2(xs.y, xs.y), sz = pack2(xs.z, xs.z), sm = pack2(xs.w, xs.w);
+    const f2 swx = pack2(ws.x, ws.x), swy = pack2(ws.y, ws.y), swz = pack2(ws.z, ws.z);
+    const f2 E = pack2(eps2, eps2), NEG3 = pack2(-3.f, -3.f);
+    const f2 sm3 = mul2(sm, NEG3), TM3 = mul2(t.TNM, NEG3);
+    const f2 dx = sub2(sx, t.TX), dy = sub2(sy, t.TY), dz = sub2(sz, t.TZ);
+    const f2 r2 = fma2(dz, dz, fma2(dy, dy, fma2(dx, dx, E)));
+    const f2 inv = rsqrt2(r2);
+    const f2 inv2 = mul2(inv, inv);
+    f2 sv = mul2(inv, inv2);
+    if (DIAG) {
+        float q0, q1;
+        unpack2(sv, q0, q1);
+        const int t0 = 128 * wib + 64 * HH + lane;
+        q0 = t0 < jj ? q0 : 0.f;
+        q1 = t0 + 32 < jj ? q1 : 0.f;
+        sv = pack2(q0, q1);
+    }
+    const f2 ux = fma2(t.TNM, swx, mul2(sm, t.TWX));
+    const f2 uy = fma2(t.TNM, swy, mul2(sm, t.TWY));
+    const f2 uz = fma2(t.TNM, swz, mul2(sm, t.TWZ));
+    const f2 dwt = fma2(dz, t.TWZ, fma2(dy, t.TWY, mul2(dx, t.TWX)));
+    const f2 dws = fma2(dz, swz, fma2(dy, swy, mul2(dx, swx)));
+    const f2 ne = mul2(inv2, fma2(sm3, dwt, mul2(TM3, dws)));
+    const f2 vx = fma2(ne, dx, ux), vy = fma2(ne, dy, uy), vz = fma2(ne, dz, uz);
+    t.NX = fma2(sv, vx, t.NX);
+    t.NY = fma2(sv, vy, t.NY);
+    t.NZ = fma2(sv, vz, t.NZ);
+    t.NG = fma2(sv, dws, t.NG);
+    PX = fma2(sv, vx, PX);
+    PY = fma2(sv, vy, PY);
+    PZ = fma2(sv, vz, PZ);
+    PG = fma2(sv, dwt, PG);
+}
+
 // One round of sym2 pair steps: lane l at step k takes source jj =
-// 32 g + (l + k) mod 32 of the staged tile against its 4 targets.  DIAG
-// masks the pairs with target index >= source index (diagonal tile).
-template <bool DIAG>
+// 32 g + (l + k) mod 32 of the staged tile against its 4 targets.  Bound by the
+// FMA pipe (math-pipe throttle at 65% of it, issue 63%): one half in scalar
+// arithmetic, twice as many targets a lane, sources staged twice against
+// register moves and fewer barriers measured the same or slower (n = 65,536:
+// 2.95, 3.00, 3.18 and 3.06 ms, this 2.94).
+template <bool DIAG, int UNROLL>
 __device__ __forceinline__ void sym2_round(const float4 *__restrict__ sxm, const float4 *__restrict__ sw,
-                                           float4 *sacc, int g, int lane, int wib, f2 EPS2, f2 NEG3,
-                                           const f2 (&TX)[2], const f2 (&TY)[2], const f2 (&TZ)[2],
-                                           const f2 (&TNM)[2], const f2 (&TWX)[2], const f2 (&TWY)[2],
-                                           const f2 (&TWZ)[2], f2 (&NX)[2], f2 (&NY)[2], f2 (&NZ)[2],
-                                           f2 (&NG)[2]) {
-    // 3 m_t for the lane's targets: d.u = m_s d.w_t - m_t d.w_s, so
-    // -3 d.u = (-3 m_s) d.w_t + (3 m_t) d.w_s from the two dot products.
-    const f2 TM3[2] = {mul2(TNM[0], NEG3), mul2(TNM[1], NEG3)};
+                                           float4 *sacc, int g, int lane, int wib, float eps2, Sym2Half &A,
+                                           Sym2Half &B) {
     // The next step's source is read one step ahead: where a block is alone on
     // its SM the read's latency was not covered (VJP and fix-up of 1,000
     // particles: 18.7 to 16.7 us; of 4,096 and more: the same).
     float4 xn = sxm[g * 32 + lane], wn = sw[g * 32 + lane];
-#pragma unroll 2
+#pragma unroll UNROLL
     for (int k = 0; k < 32; ++k) {
         const int jj = g * 32 + ((lane + k) & 31), jn = g * 32 + ((lane + k + 1) & 31);
         const float4 xs = xn, ws = wn;
         xn = sxm[jn];
         wn = sw[jn];
-        const f2 sx = pack2(xs.x, xs.x), sy = pack2(xs.y, xs.y), sz = pack2(xs.z, xs.z);
-        const f2 sm = pack2(xs.w, xs.w);
-        const f2 sm3 = mul2(sm, NEG3);
-        const f2 swx = pack2(ws.x, ws.x), swy = pack2(ws.y, ws.y), swz = pack2(ws.z, ws.z);
         f2 PX = 0ull, PY = 0ull, PZ = 0ull, PG = 0ull;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const f2 dx = sub2(sx, TX[h]), dy = sub2(sy, TY[h]), dz = sub2(sz, TZ[h]);
-            const f2 r2 = fma2(dz, dz, fma2(dy, dy, fma2(dx, dx, EPS2)));
-            const f2 inv = rsqrt2(r2);
-            const f2 inv2 = mul2(inv, inv);
-            f2 sv = mul2(inv, inv2);
-            if (DIAG) {
-                // Target index 128 w + 64 h + 32 e + lane < source index jj.
-                float s0, s1;
-                unpack2(sv, s0, s1);
-                const int t0 = 128 * wib + 64 * h + lane;
-                s0 = t0 < jj ? s0 : 0.f;
-                s1 = t0 + 32 < jj ? s1 : 0.f;
-                sv = pack2(s0, s1);
-            }
-            // u = m_s w_t - m_t w_s; v = u - 3 inv2 (d.u) d.
-            const f2 ux = fma2(TNM[h], swx, mul2(sm, TWX[h]));
-            const f2 uy = fma2(TNM[h], swy, mul2(sm, TWY[h]));
-            const f2 uz = fma2(TNM[h], swz, mul2(sm, TWZ[h]));
-            const f2 dwt = fma2(dz, TWZ[h], fma2(dy, TWY[h], mul2(dx, TWX[h])));
-            const f2 dws = fma2(dz, swz, fma2(dy, swy, mul2(dx, swx)));
-            const f2 ne = mul2(inv2, fma2(sm3, dwt, mul2(TM3[h], dws)));  // -3 inv2 d.u
-            const f2 vx = fma2(ne, dx, ux), vy = fma2(ne, dy, uy), vz = fma2(ne, dz, uz);
-            NX[h] = fma2(sv, vx, NX[h]);
-            NY[h] = fma2(sv, vy, NY[h]);
-            NZ[h] = fma2(sv, vz, NZ[h]);
-            NG[h] = fma2(sv, dws, NG[h]);
-            PX = fma2(sv, vx, PX);
-            PY = fma2(sv, vy, PY);
-            PZ = fma2(sv, vz, PZ);
-            PG = fma2(sv, dwt, PG);
-        }
+        sym2_half<DIAG, 0>(A, xs, ws, jj, lane, wib, eps2, PX, PY, PZ, PG);
+        sym2_half<DIAG, 1>(B, xs, ws, jj, lane, wib, eps2, PX, PY, PZ, PG);
         float4 acc = sacc[jj];
         float lo, hi;
         unpack2(PX, lo, hi);
@@ -472,20 +480,21 @@ __device__ __forceinline__ void sym2_round(const float4 *__restrict__ sxm, const
 template <int Q, int TILE>
 __global__ void __launch_bounds__(SYM2_WARPS<TILE> * 32, 16 / SYM2_WARPS<TILE>) adjoint_vjp_sym2_kernel(Sym2Args a) {
     constexpr int WARPS = SYM2_WARPS<TILE>, G = TILE / 32 / Q, SPAN = G * 32;
+    // Steps unrolled: 4,096 particles 26.7 us with 2, 25.4 with 3; 65,536: 2.94 ms, 3.01.
+    constexpr int UNROLL = TILE == SYM2_SMALL_T ? 3 : 2;
     static_assert(G >= WARPS, "each warp of a round takes its own source group");
     __shared__ float4 sxm[TILE], sw[TILE], sacc[TILE];
     __shared__ long long s_unit;
     __shared__ int s_gend, s_ntgt;  // source groups and targets of the unit that hold particles
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, tid = threadIdx.x;
     const int64_t NU = a.NU;
-    const f2 EPS2 = pack2(a.eps2, a.eps2), NEG3 = pack2(-3.f, -3.f);
     if (tid == 0) s_unit = -1;
     for (;;) {
         __syncthreads();  // the previous unit is done with s_unit and shared memory
         if (tid == 0)
             s_unit = a.counter ? (long long)atomicAdd(a.counter, 1ull) : s_unit < 0 ? (long long)blockIdx.x : (long long)NU;
         __syncthreads();
-        f2 TX[2], TY[2], TZ[2], TNM[2], TWX[2], TWY[2], TWZ[2], NX[2], NY[2], NZ[2], NG[2];
+        Sym2Half half[2];
         bool diag;
         int gbase;
         {
@@ -515,14 +524,15 @@ __global__ void __launch_bounds__(SYM2_WARPS<TILE> * 32, 16 / SYM2_WARPS<TILE>) 
                 x[e] = i < a.n ? __ldg(a.xm + i) : make_float4(0.f, 0.f, 0.f, 0.f);
                 w[e] = sym2_w(a, i);
             }
-            TX[h] = pack2(x[0].x, x[1].x);
-            TY[h] = pack2(x[0].y, x[1].y);
-            TZ[h] = pack2(x[0].z, x[1].z);
-            TNM[h] = pack2(-x[0].w, -x[1].w);
-            TWX[h] = pack2(w[0].x, w[1].x);
-            TWY[h] = pack2(w[0].y, w[1].y);
-            TWZ[h] = pack2(w[0].z, w[1].z);
-            NX[h] = NY[h] = NZ[h] = NG[h] = 0ull;
+            Sym2Half &q = half[h];
+            q.TX = pack2(x[0].x, x[1].x);
+            q.TY = pack2(x[0].y, x[1].y);
+            q.TZ = pack2(x[0].z, x[1].z);
+            q.TNM = pack2(-x[0].w, -x[1].w);
+            q.TWX = pack2(w[0].x, w[1].x);
+            q.TWY = pack2(w[0].y, w[1].y);
+            q.TWZ = pack2(w[0].z, w[1].z);
+            q.NX = q.NY = q.NZ = q.NG = 0ull;
         }
         // Stage the slice's sources (tile-local indices sl*SPAN .. +SPAN-1).
         for (int t = tid; t < SPAN; t += WARPS * 32) {
@@ -541,11 +551,9 @@ __global__ void __launch_bounds__(SYM2_WARPS<TILE> * 32, 16 / SYM2_WARPS<TILE>) 
             // Warp-uniform branches; every warp still reaches the barrier.
             if (128 * wib < s_ntgt && g < s_gend) {
                 if (!diag)
-                    sym2_round<false>(sxm, sw, sacc, g, lane, wib, EPS2, NEG3, TX, TY, TZ, TNM, TWX, TWY, TWZ, NX,
-                                      NY, NZ, NG);
+                    sym2_round<false, UNROLL>(sxm, sw, sacc, g, lane, wib, a.eps2, half[0], half[1]);
                 else if (4 * wib <= g)
-                    sym2_round<true>(sxm, sw, sacc, g, lane, wib, EPS2, NEG3, TX, TY, TZ, TNM, TWX, TWY, TWZ, NX,
-                                     NY, NZ, NG);
+                    sym2_round<true, UNROLL>(sxm, sw, sacc, g, lane, wib, a.eps2, half[0], half[1]);
             }
             __syncthreads();
         }
@@ -559,10 +567,10 @@ __global__ void __launch_bounds__(SYM2_WARPS<TILE> * 32, 16 / SYM2_WARPS<TILE>) 
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             float x0, x1, y0, y1, z0, z1, g0, g1;
-            unpack2(NX[h], x0, x1);
-            unpack2(NY[h], y0, y1);
-            unpack2(NZ[h], z0, z1);
-            unpack2(NG[h], g0, g1);
+            unpack2(half[h].NX, x0, x1);
+            unpack2(half[h].NY, y0, y1);
+            unpack2(half[h].NZ, z0, z1);
+            unpack2(half[h].NG, g0, g1);
             float4 *row = a.rowpart + u * TILE + 128 * wib + 64 * h + lane;
             row[0] = make_float4(-x0, -y0, -z0, -g0);
             row[32] = make_float4(-x1, -y1, -z1, -g1);
