@@ -35,7 +35,7 @@
 namespace gb {
 
 constexpr int DS_T = SYM_TILE;
-constexpr int DS_K_UNROLL = 4;  // steps of a round unrolled (1-4 measured within 3%)
+constexpr int DS_K_UNROLL = 4;  // steps of a potential round unrolled (1-4 measured within 3%)
 constexpr int DS_ACC = 0, DS_KDK = 1, DS_PHI = 2;
 
 // CTA shape for H packed target pairs per lane (2H targets): 8/H warps
@@ -105,7 +105,11 @@ __device__ __forceinline__ void ds_round(const float4 *__restrict__ sxm, float4 
     // 8.1 to 6.3 us, 4,096: 10.2 to 9.4, 6,144: 16.9 to 15.8).  The large shape
     // has 16 warps an SM for that and no registers left.
     float4 xn = sxm[g * 32 + lane];
-#pragma unroll DS_K_UNROLL
+    // Steps unrolled, 4 / 2, force kernel: large shape 12,000: 55.8 / 50.5 us,
+    // 20,000: 125 / 123 (with the potential 146 / 139), 262,144: the same; small
+    // tiles 1,000: 6.3 / 7.0, 4,096: 9.4 / 9.8.
+    constexpr int UNROLL = H == DS_SMALL_H ? 4 : 2;
+#pragma unroll UNROLL
     for (int k = 0; k < 32; ++k) {
         const int jj = g * 32 + ((lane + k) & 31);
         const float4 xs = H == DS_SMALL_H ? xn : sxm[jj];
