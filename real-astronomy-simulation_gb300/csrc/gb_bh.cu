@@ -298,8 +298,11 @@ __device__ __forceinline__ float size2_of(const NodeSum &s) {
 // ranges: 59 / 155; nodes of a chunk in queued rounds, records inside: 47 /
 // 168; records apart: 27 / 129; one thread per leaf upwards instead of
 // rounds: 24 / 122; rounds down to 32 nodes: 20 / 105; 4 CTAs per SM (64
-// registers): 20 / 102.  128 threads: 27 / 110; 512: 18 / 152.
-constexpr int TREE_THREADS = 256;
+// registers): 20 / 102.  128 threads: 27 / 110; 512, one CTA per SM: 18 / 152.
+// So 512 threads while every unit has an SM of its own (77,824 leaves on 152
+// SMs; tree stage, 256 / 512: 500: 15.0 / 12.6; 10,000: 24.6 / 22.7; 20,000:
+// 35.4 / 30.9; 60,000: 35.8 / 31.6; 80,000: 37.9 / 39.3; 300,000: 47.8 / 58.8).
+constexpr int TREE_THREADS = 256, TREE_WIDE = 512;  // per CTA; TREE_WIDE while every unit has an SM of its own
 constexpr int TREE_CHUNK = 512;   // leaves or subtrees joined at a time
 constexpr int TREE_GROUP = 32;    // units of a level that the next one joins (one per lane)
 constexpr int TREE_PEND = 192;    // subtrees left of a unit (63 key bits + 31 index bits on each side)
@@ -388,7 +391,7 @@ struct TreeShared {
     unsigned queue[2][TREE_CHUNK / 2];        // nodes to make: first item | last item << 10 | split << 20
     int queued[3];
     short end[TREE_CHUNK];
-    int scan[TREE_THREADS / 32];
+    int scan[TREE_CHUNK / 32];
     int before[TREE_GROUP + 1];               // subtrees of the units before each one of a group
     bool last_unit;
 
@@ -431,15 +434,16 @@ __device__ __forceinline__ bool tree_make(TreeShared &w, int a, int b, int j, bo
 
 // Joins the m items in w (summaries, leaf ranges, deltas; m >= 1) as far as
 // they reach.  Complete after the barrier at its end.
+template <int THREADS>
 __device__ __forceinline__ void tree_join(TreeShared &w, int m) {
     const int tid = threadIdx.x;
-    for (int i = tid; i <= m; i += TREE_THREADS) w.came[i] = 0u;
+    for (int i = tid; i <= m; i += THREADS) w.came[i] = 0u;
     if (tid < 3) w.queued[tid] = 0;
     __syncthreads();
     auto push = [&](int a, int b, int j, int q, int c) {
         w.queue[q][atomicAdd(&w.queued[c], 1)] = (unsigned)a | (unsigned)b << 10 | (unsigned)j << 20;
     };
-    for (int i = tid; i < m; i += TREE_THREADS) {
+    for (int i = tid; i < m; i += THREADS) {
         int a = i, b = i, j;
         const int da = w.delta[i], db = w.delta[i + 1];
         if ((da >= 0 || db >= 0) && tree_come(w, db > da, a, b, j)) push(a, b, j, 0, 0);
@@ -450,7 +454,7 @@ __device__ __forceinline__ void tree_join(TreeShared &w, int m) {
         const int ready = w.queued[c], c1 = c == 2 ? 0 : c + 1;
         if (ready <= 32) break;
         if (tid == 0) w.queued[c1 == 2 ? 0 : c1 + 1] = 0;  // read one round ago, used by the next one
-        for (int i = tid; i < ready; i += TREE_THREADS) {
+        for (int i = tid; i < ready; i += THREADS) {
             const unsigned e = w.queue[q][i];
             int a = (int)(e & 1023u), b = (int)(e >> 10 & 1023u), j = (int)(e >> 20);
             bool left;
@@ -473,9 +477,9 @@ __device__ __forceinline__ void tree_join(TreeShared &w, int m) {
 // The records of the nodes that tree_join made; base(i): the summary of item
 // i.  Apart from the joining, because the divisions of the centres and the 13
 // stores of a node would lengthen every level.
-template <typename F>
+template <int THREADS, typename F>
 __device__ __forceinline__ void tree_records(const TreeShared &w, const TreeArgs &t, int m, F base) {
-    for (int j = threadIdx.x + 1; j < m; j += TREE_THREADS) {
+    for (int j = threadIdx.x + 1; j < m; j += THREADS) {
         const int a = (int)(w.came[j] & 0xFFFFu) - 1, b = (int)(w.came[j] >> 16) - 1;
         if (a < 0 || b < 0) continue;
         const int da = w.delta[a], db = w.delta[b + 1], l = w.first[a], r = w.last[b];
@@ -486,12 +490,13 @@ __device__ __forceinline__ void tree_records(const TreeShared &w, const TreeArgs
 }
 
 // Writes the subtrees that are left, in leaf order, to dst; returns how many.
+template <int THREADS>
 __device__ __forceinline__ int tree_left(TreeShared &w, TreeItem *dst, int m) {
-    constexpr int PER = TREE_CHUNK / TREE_THREADS;
+    constexpr int PER = TREE_CHUNK / THREADS;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    for (int i = tid; i < TREE_CHUNK; i += TREE_THREADS) w.end[i] = 0;  // 1 + the last item of the subtree from here
+    for (int i = tid; i < TREE_CHUNK; i += THREADS) w.end[i] = 0;  // 1 + the last item of the subtree from here
     __syncthreads();
-    for (int j = tid; j <= m; j += TREE_THREADS) {
+    for (int j = tid; j <= m; j += THREADS) {
         const int a = (int)(w.came[j] & 0xFFFFu) - 1, b = (int)(w.came[j] >> 16) - 1;
         if (a >= 0 && b < 0) w.end[a] = (short)j;
         else if (b >= 0 && a < 0) w.end[j] = (short)(b + 1);
@@ -510,7 +515,7 @@ __device__ __forceinline__ int tree_left(TreeShared &w, TreeItem *dst, int m) {
     __syncthreads();
     int at = inc - own, total = 0;
 #pragma unroll
-    for (int k = 0; k < TREE_THREADS / 32; ++k) {
+    for (int k = 0; k < THREADS / 32; ++k) {
         if (k < wid) at += w.scan[k];
         total += w.scan[k];
     }
@@ -548,13 +553,14 @@ __device__ __forceinline__ TreeItem load_item(const TreeItem *p) {  // written b
     return u.x;
 }
 
-template <typename KeyT>
-__global__ void __launch_bounds__(TREE_THREADS, 4) bh_tree_kernel(const KeyT *__restrict__ keys, TreeArgs t) {
+template <typename KeyT, int THREADS>
+__global__ void __launch_bounds__(THREADS, THREADS == TREE_WIDE ? 1 : 4)
+bh_tree_kernel(const KeyT *__restrict__ keys, TreeArgs t) {
     __shared__ TreeShared w;
     const int tid = threadIdx.x, n = t.n;
     int unit = blockIdx.x, units = gridDim.x, base = 0, groups = 0;  // units and groups of the levels below
     int m = min(TREE_CHUNK, n - unit * TREE_CHUNK);
-    for (int i = tid; i <= m; i += TREE_THREADS) {
+    for (int i = tid; i <= m; i += THREADS) {
         const int g = unit * TREE_CHUNK + i;
         w.delta[i] = g >= 1 ? (signed char)kdelta(keys, n, g - 1, g) : (signed char)-1;
         if (i == m) continue;
@@ -576,9 +582,9 @@ __global__ void __launch_bounds__(TREE_THREADS, 4) bh_tree_kernel(const KeyT *__
         return;
     }
     __syncthreads();
-    tree_join(w, m);
+    tree_join<THREADS>(w, m);
     if (units == 1) {
-        tree_records(w, t, m, [&](int i) { return leaf_sum(w.leaf[i]); });
+        tree_records<THREADS>(w, t, m, [&](int i) { return leaf_sum(w.leaf[i]); });
         return;
     }
     TreeItem *items = nullptr;  // the items of levels above the leaves
@@ -593,7 +599,7 @@ __global__ void __launch_bounds__(TREE_THREADS, 4) bh_tree_kernel(const KeyT *__
     };
     auto above = [&](int i) { return load_item(item(i)).s; };
     for (int level = 0; units > 1; ++level) {
-        const int left = tree_left(w, t.items + (int64_t)(base + unit) * TREE_PEND, m);
+        const int left = tree_left<THREADS>(w, t.items + (int64_t)(base + unit) * TREE_PEND, m);
         // The last unit of the group to finish goes on with all of its
         // subtrees; the records are written while that is being found out.
         static_assert(TREE_GROUP == 32, "one unit of a group per lane");
@@ -604,8 +610,8 @@ __global__ void __launch_bounds__(TREE_THREADS, 4) bh_tree_kernel(const KeyT *__
             __threadfence();
             w.last_unit = atomicAdd(t.done + groups + group, 1u) == (unsigned)(gn - 1);
         }
-        if (level == 0) tree_records(w, t, m, [&](int i) { return leaf_sum(w.leaf[i]); });
-        else tree_records(w, t, m, above);
+        if (level == 0) tree_records<THREADS>(w, t, m, [&](int i) { return leaf_sum(w.leaf[i]); });
+        else tree_records<THREADS>(w, t, m, above);
         __syncthreads();
         if (!w.last_unit) return;
         __threadfence();
@@ -631,12 +637,12 @@ __global__ void __launch_bounds__(TREE_THREADS, 4) bh_tree_kernel(const KeyT *__
             for (int i0 = 0; i0 < total; i0 += TREE_CHUNK) {
                 m = min(TREE_CHUNK, total - i0);
                 __syncthreads();
-                for (int i = tid; i < m; i += TREE_THREADS) tree_take(w, load_item(item(i0 + i)), i, i == m - 1);
+                for (int i = tid; i < m; i += THREADS) tree_take(w, load_item(item(i0 + i)), i, i == m - 1);
                 __syncthreads();
-                tree_join(w, m);
-                tree_records(w, t, m, [&](int i) { return load_item(item(i0 + i)).s; });
+                tree_join<THREADS>(w, m);
+                tree_records<THREADS>(w, t, m, [&](int i) { return load_item(item(i0 + i)).s; });
                 __syncthreads();  // the items are read
-                out += tree_left(w, items + out, m);
+                out += tree_left<THREADS>(w, items + out, m);
             }
             __syncthreads();
             __threadfence();
@@ -645,15 +651,15 @@ __global__ void __launch_bounds__(TREE_THREADS, 4) bh_tree_kernel(const KeyT *__
         }
         __syncthreads();
         m = total;
-        for (int i = tid; i < m; i += TREE_THREADS) tree_take(w, load_item(item(i)), i, i == m - 1);
+        for (int i = tid; i < m; i += THREADS) tree_take(w, load_item(item(i)), i, i == m - 1);
         __syncthreads();
-        tree_join(w, m);
+        tree_join<THREADS>(w, m);
         base += units;
         groups += (units + TREE_GROUP - 1) / TREE_GROUP;
         unit = group;
         units = (units + TREE_GROUP - 1) / TREE_GROUP;
     }
-    tree_records(w, t, m, above);
+    tree_records<THREADS>(w, t, m, above);
 }
 
 // Units and groups of all levels for n leaves.
@@ -911,8 +917,10 @@ static int build_tree(gb_bh_t *h, const float4 *xm, const uint32_t *order, int64
     t.root = h->root;
     t.gsize = groups ? h->gsize : nullptr;
     t.diag = h->diag;
-    bh_tree_kernel<KeyT><<<(unsigned)((n + TREE_CHUNK - 1) / TREE_CHUNK), TREE_THREADS, 0, s>>>(
-        (const KeyT *)h->keys[h->cur], t);
+    const unsigned grid = (unsigned)((n + TREE_CHUNK - 1) / TREE_CHUNK);
+    const KeyT *keys = (const KeyT *)h->keys[h->cur];
+    if (grid <= (unsigned)h->sms) bh_tree_kernel<KeyT, TREE_WIDE><<<grid, TREE_WIDE, 0, s>>>(keys, t);
+    else bh_tree_kernel<KeyT, TREE_THREADS><<<grid, TREE_THREADS, 0, s>>>(keys, t);
     GB_CUDA_TRY(cudaGetLastError());
     h->groups_n = groups ? n : -1;
     h->launches += 1;

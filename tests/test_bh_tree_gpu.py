@@ -97,3 +97,14 @@ def test_groups_marked_after_the_build(cuda_dev, n):
         assert b.diag()["bad_tree"] == 0
         b.close()
     assert torch.equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("extra", [0, 1])
+def test_tree_at_the_change_of_block_size(cuda_dev, orc, extra):
+    """One chunk per SM is the last size of the wide blocks."""
+    ic = importlib.import_module(PKG_NAME + ".ic")
+    n = 512 * torch.cuda.get_device_properties(cuda_dev).multi_processor_count + extra
+    pos, _, mass = ic.plummer(n, seed=n)
+    pos, mass = (a.astype(np.float32).astype(np.float64) for a in (pos, mass))
+    b, _ = _check_tree(cuda_dev, orc, pos, mass, 21)
+    b.close()
