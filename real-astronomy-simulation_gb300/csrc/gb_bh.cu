@@ -754,9 +754,10 @@ struct gb_bh {
     int64_t n_max;
     int key_bits;
     int64_t n;  // n of the last build (-1: none)
+    // Radix ping-pong.  Every sort ends in pair 0, whatever n is: a replayed
+    // graph sorts again without passing through the host code.
     void *keys[2];
     uint32_t *vals[2];
-    int cur;  // which buffer holds the sorted result
     uint32_t *sort_scratch;  // radix_scratch_size(n_max) words
     float4 *bbox_part;
     int bbox_blocks;
@@ -848,7 +849,6 @@ extern "C" int gb_bh_create(gb_bh_t **out, int64_t n_max, int key_bits) {
     h->tpl = -1;
     h->use_graph = 1;
     h->n = -1;
-    h->cur = 0;
     const int64_t nn = n_max, ni = std::max<int64_t>(n_max - 1, 1), nodes = 2 * n_max;
     h->bbox_blocks = std::max(1, std::min(h->sms * 4, (int)((n_max + BBOX_THREADS - 1) / BBOX_THREADS)));
     bool ok = true;
@@ -918,7 +918,7 @@ static int build_tree(gb_bh_t *h, const float4 *xm, const uint32_t *order, int64
     t.gsize = groups ? h->gsize : nullptr;
     t.diag = h->diag;
     const unsigned grid = (unsigned)((n + TREE_CHUNK - 1) / TREE_CHUNK);
-    const KeyT *keys = (const KeyT *)h->keys[h->cur];
+    const KeyT *keys = (const KeyT *)h->keys[0];
     if (grid <= (unsigned)h->sms) bh_tree_kernel<KeyT, TREE_WIDE><<<grid, TREE_WIDE, 0, s>>>(keys, t);
     else bh_tree_kernel<KeyT, TREE_THREADS><<<grid, TREE_THREADS, 0, s>>>(keys, t);
     GB_CUDA_TRY(cudaGetLastError());
@@ -934,6 +934,7 @@ static int build_impl(gb_bh_t *h, float4 *xm, float4 *vel, const float4 *acc, in
     const int nblk = std::max(1, std::min(h->bbox_blocks, (int)((n + BBOX_THREADS - 1) / BBOX_THREADS)));
     // The sort's scratch, the tree's finished units and the group walk's marks.
     constexpr int passes = (3 * BITS + 7) / 8;
+    static_assert(passes % 2 == 0, "the sorted keys are in pair 0");
     const bool groups = h->tpl == 3, small = radix_small(n, passes);
     int64_t units, ngroups;
     tree_units(n, &units, &ngroups);
@@ -948,16 +949,16 @@ static int build_impl(gb_bh_t *h, float4 *xm, float4 *vel, const float4 *acc, in
     KeyT *kk[2] = {(KeyT *)h->keys[0], (KeyT *)h->keys[1]};
     if (small) {
         mark(h, slot, 1, s);
-        h->cur = radix_sort_small<KeyT>(MortonKey<KeyT, BITS>{xm, h->prm}, kk, h->vals, n, s);
+        radix_sort_small<KeyT>(MortonKey<KeyT, BITS>{xm, h->prm}, kk, h->vals, n, s);
     } else {
         const unsigned gk = std::min((unsigned)(h->sms * 4), (unsigned)((n + KEY_THREADS - 1) / KEY_THREADS));
         bh_morton_kernel<KeyT, BITS><<<gk, KEY_THREADS, 0, s>>>(xm, n, h->prm, kk[0], h->sort_scratch);
         mark(h, slot, 1, s);
-        h->cur = radix_sort_counted<KeyT>(kk, h->vals, n, passes, h->sort_scratch, h->diag, s);
+        radix_sort_counted<KeyT>(kk, h->vals, n, passes, h->sort_scratch, h->diag, s);
     }
     mark(h, slot, 2, s);
     // The group walk's groups are marked when the handle walks groups.
-    GB_TRY(build_tree<KeyT>(h, xm, h->vals[h->cur], n, groups, s));
+    GB_TRY(build_tree<KeyT>(h, xm, h->vals[0], n, groups, s));
     mark(h, slot, 3, s);
     GB_CUDA_TRY(cudaGetLastError());
     mark(h, slot, 4, s);
@@ -1045,7 +1046,7 @@ static int traverse(gb_bh_t *h, float4 *acc, float4 *vel, float *phi, float thet
     a.leaf = h->leaf;
     a.inode = h->inode;
     a.root = h->root;
-    a.order = h->vals[h->cur];
+    a.order = h->vals[0];
     a.acc = acc;
     a.vel = vel;
     a.n = (int)n;
@@ -1371,10 +1372,10 @@ extern "C" int gb_bh_export(gb_bh_t *h, int what, void *dst, void *stream) {
     const unsigned grid = (unsigned)((count + 255) / 256);
     cudaStream_t s = (cudaStream_t)stream;
     if (h->key_bits == 10)
-        bh_export_kernel<uint32_t><<<grid, 256, 0, s>>>(what, n, (const uint32_t *)h->keys[h->cur], h->vals[h->cur],
+        bh_export_kernel<uint32_t><<<grid, 256, 0, s>>>(what, n, (const uint32_t *)h->keys[0], h->vals[0],
                                                         h->child, h->parent, h->leaf, h->sums, h->bmin, h->bmax, dst);
     else
-        bh_export_kernel<uint64_t><<<grid, 256, 0, s>>>(what, n, (const uint64_t *)h->keys[h->cur], h->vals[h->cur],
+        bh_export_kernel<uint64_t><<<grid, 256, 0, s>>>(what, n, (const uint64_t *)h->keys[0], h->vals[0],
                                                         h->child, h->parent, h->leaf, h->sums, h->bmin, h->bmax, dst);
     GB_CUDA_TRY(cudaGetLastError());
     return GB_OK;

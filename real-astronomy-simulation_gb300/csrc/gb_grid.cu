@@ -429,7 +429,7 @@ extern "C" int gb_grid_rebuild(gb_grid_t *h, const float *xm, const float *hsml,
         const CellKey key{(const float4 *)xm, is_star, h->geom};
         int cur = 0;
         if (small) {
-            cur = radix_sort_small<uint32_t>(key, h->keys, h->vals, n, s);
+            radix_sort_small<uint32_t>(key, h->keys, h->vals, n, s);
         } else {
             grid_key_kernel<<<nblk, GRID_THREADS, 0, s>>>(key, n, h->keys[0], h->sort_scratch, h->passes);
             cur = radix_sort_counted<uint32_t>(h->keys, h->vals, n, h->passes, h->sort_scratch, h->diag, s);

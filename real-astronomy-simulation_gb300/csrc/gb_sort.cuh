@@ -556,20 +556,20 @@ inline bool radix_small(int64_t n, int passes) {
 // Kernels of such a sort.
 inline int radix_small_launches(int64_t n) { return n <= SS_BLOCK ? 1 : n <= SS_ONE_N ? 2 : 3; }
 
-// Sorts the keys src(0 .. n - 1) with their indices; returns the index of the
-// pair of k and v that holds the result.
+// Sorts the keys src(0 .. n - 1) with their indices.  The result is in k[0] and
+// v[0] whatever n is, like that of an even number of digits: two kernels start
+// in the other pair.
 template <typename KeyT, typename Source>
-static int radix_sort_small(const Source &src, KeyT *k[2], uint32_t *v[2], int64_t n, cudaStream_t s) {
-    const int launches = radix_small_launches(n);
+static void radix_sort_small(const Source &src, KeyT *k[2], uint32_t *v[2], int64_t n, cudaStream_t s) {
+    const int launches = radix_small_launches(n), a = launches == 2 ? 1 : 0, b = a ^ 1;
     const unsigned gr = (unsigned)((n + SS_KEYS - 1) / SS_KEYS);
-    ss_block_kernel<KeyT, Source><<<(unsigned)((n + SS_BLOCK - 1) / SS_BLOCK), SS_BLOCK, 0, s>>>(src, (int)n, k[0],
-                                                                                               v[0]);
+    ss_block_kernel<KeyT, Source><<<(unsigned)((n + SS_BLOCK - 1) / SS_BLOCK), SS_BLOCK, 0, s>>>(src, (int)n, k[a],
+                                                                                               v[a]);
     if (launches > 1)
-        ss_group_kernel<KeyT><<<gr, SS_KEYS, 0, s>>>(k[0], v[0], (int)n, launches == 2 ? 32 : (int)SS_GROUP, k[1],
-                                                     v[1]);
+        ss_group_kernel<KeyT><<<gr, SS_KEYS, 0, s>>>(k[a], v[a], (int)n, launches == 2 ? 32 : (int)SS_GROUP, k[b],
+                                                     v[b]);
     if (launches > 2)
         ss_merge_kernel<KeyT><<<gr, SS_KEYS, 0, s>>>(k[1], v[1], (int)n, (int)(SS_GROUP * SS_BLOCK), k[0], v[0]);
-    return launches == 2 ? 1 : 0;
 }
 
 // Scratch words that are zero when the kernel that makes the keys starts:
