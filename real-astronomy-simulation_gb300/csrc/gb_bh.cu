@@ -801,6 +801,7 @@ struct gb_bh {
         }
     } gkey[2];
     uint64_t graph_launches[2];  // kernels in each captured step
+    int64_t graph_groups[2];     // groups_n after each captured step
     double2 *epart;              // energy block partials (gb_bh_energy)
     int epart_cap;
     int *gsize;                  // group-walk groups of the last build (mode 3)
@@ -1217,10 +1218,16 @@ static int ensure_graph(gb_bh_t *h, int g, const gb_bh::Key &key, float4 *x, flo
     if (h->gexec[g]) cudaGraphExecDestroy(h->gexec[g]);
     h->gexec[g] = nullptr;
     GB_CUDA_TRY(cudaStreamBeginCapture(h->gstream, cudaStreamCaptureModeThreadLocal));
+    // What a step leaves on the handle is true once it has run: it is noted
+    // here and set after the replay.
     const uint64_t l0 = h->launches;
+    const int64_t n0 = h->n, groups0 = h->groups_n;
     const int st = kdk_step(h, x, v, a, phi, n, theta, eps2, G, dt, max_stack, h->gstream);
     h->graph_launches[g] = h->launches - l0;
+    h->graph_groups[g] = h->groups_n;
     h->launches = l0;
+    h->n = n0;
+    h->groups_n = groups0;
     cudaGraph_t graph = nullptr;
     const cudaError_t e = cudaStreamEndCapture(h->gstream, &graph);
     if (st != GB_OK) {
@@ -1275,6 +1282,7 @@ static int bh_kdk_impl(gb_bh_t *h, float *xm, float *vel, float *acc, float *phi
     GB_CUDA_TRY(cudaStreamWaitEvent(s, h->gev_out, 0));
     h->launches += h->graph_launches[0] * (uint64_t)plain_steps + (phi ? h->graph_launches[1] : 0);
     h->n = n;
+    h->groups_n = h->graph_groups[phi ? 1 : 0];  // of the step replayed last
     return h->check ? check_failures(h, s, call) : GB_OK;
 }
 

@@ -87,3 +87,30 @@ def test_steps_with_and_without_potential_at_two_sizes(cuda_dev, n, n_phi):
         assert torch.equal(phi, phi_ref)
     for h in (b, ref, ref_phi):
         h.close()
+
+
+@pytest.mark.parametrize("replayed", [-1, 3])
+def test_groups_after_a_replay(cuda_dev, replayed):
+    """The group walk after a replayed step walks that step's groups, whichever
+    shape the step had and the build before it."""
+    n = 20000
+    b = _handle(cuda_dev, n, 21, True)
+    ref = _handle(cuda_dev, n, 21, False)
+    s, s_ref, between = _state(cuda_dev, n, 5), _state(cuda_dev, n, 5), _state(cuda_dev, n, 6)
+    b.set_traversal(replayed)
+    ref.set_traversal(replayed)
+    b.kdk(*s, DT)  # captured
+    b.set_traversal(2 - replayed)  # 3 and -1
+    b.compute(between[0], between[2])
+    b.set_traversal(replayed)
+    b.kdk(*s, DT)  # replayed
+    ref.kdk(*s_ref, DT, 2)
+    out = []
+    for h, x in ((b, s[0]), (ref, s_ref[0])):
+        h.set_traversal(3)
+        acc = torch.zeros_like(x)
+        h.accel(acc)
+        out.append(acc)
+        assert h.diag()["bad_tree"] == 0
+        h.close()
+    assert torch.equal(s[0], s_ref[0]) and torch.equal(out[0], out[1])
