@@ -524,6 +524,15 @@ uint64_t gb_grid_launch_count(gb_grid_t *h);
 int gb_sort_wait_probe(int spin_limit, int publish_first, uint32_t *excl_out,
                        uint64_t *timeouts_out);
 
+/* Test support for the tree kernel's bounds: builds the tree of n particles
+ * over the given keys (device, n uint32 for key_bits 10, n uint64 for 21) and
+ * order (device, particle of each leaf) as they are, without sorting.  Keys out
+ * of order, which otherwise only an expired wait of the sort could leave, make
+ * bad_tree grow; everything stays inside the handle's arrays.  Asynchronous.
+ * No reference counterpart. */
+int gb_bh_tree_probe(gb_bh_t *h, const float *xm, const void *keys,
+                     const uint32_t *order, int64_t n, void *stream);
+
 /* ------------------------------------------------------------ calibration */
 /* Launches an FP32 FMA-throughput kernel (packed = 1: .f32x2 form) on
  * `stream`; *flops receives the FLOP count of the launch, which the caller

@@ -305,7 +305,12 @@ __device__ __forceinline__ float size2_of(const NodeSum &s) {
 constexpr int TREE_THREADS = 256, TREE_WIDE = 512;  // per CTA; TREE_WIDE while every unit has an SM of its own
 constexpr int TREE_CHUNK = 512;   // leaves or subtrees joined at a time
 constexpr int TREE_GROUP = 32;    // units of a level that the next one joins (one per lane)
-constexpr int TREE_PEND = 192;    // subtrees left of a unit (63 key bits + 31 index bits on each side)
+// Subtrees left of a unit: in sorted keys the common prefix grows from one to
+// the next up to the longest and falls again, so 63 key bits + 31 index bits on
+// each side.  Keys out of order, which an expired wait of the sort can leave,
+// may keep any number apart (alternating ones all 512): those past the bound are
+// dropped and counted as bad_tree.
+constexpr int TREE_PEND = 192;
 // Leaves per group of the group walk (traversal shape 3).
 constexpr int GW_GROUP = 32;
 
@@ -489,9 +494,10 @@ __device__ __forceinline__ void tree_records(const TreeShared &w, const TreeArgs
     }
 }
 
-// Writes the subtrees that are left, in leaf order, to dst; returns how many.
+// Writes the subtrees that are left, in leaf order, to dst; returns how many,
+// TREE_PEND at most.
 template <int THREADS>
-__device__ __forceinline__ int tree_left(TreeShared &w, TreeItem *dst, int m) {
+__device__ __forceinline__ int tree_left(TreeShared &w, TreeItem *dst, int m, unsigned long long *diag) {
     constexpr int PER = TREE_CHUNK / THREADS;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     for (int i = tid; i < TREE_CHUNK; i += THREADS) w.end[i] = 0;  // 1 + the last item of the subtree from here
@@ -529,9 +535,12 @@ __device__ __forceinline__ int tree_left(TreeShared &w, TreeItem *dst, int m) {
         x.s = w.get(x.dr > x.dl ? b : a);
         x.l = w.first[a];
         x.r = w.last[b];
-        dst[at++] = x;
+        if (at < TREE_PEND) dst[at] = x;
+        ++at;
     }
-    return total;
+    if (total <= TREE_PEND) return total;
+    if (tid == 0) atomicAdd(diag + DIAG_BAD_TREE, (unsigned long long)(total - TREE_PEND));
+    return TREE_PEND;
 }
 
 __device__ __forceinline__ void tree_take(TreeShared &w, const TreeItem &x, int i, bool last) {
@@ -599,7 +608,7 @@ bh_tree_kernel(const KeyT *__restrict__ keys, TreeArgs t) {
     };
     auto above = [&](int i) { return load_item(item(i)).s; };
     for (int level = 0; units > 1; ++level) {
-        const int left = tree_left<THREADS>(w, t.items + (int64_t)(base + unit) * TREE_PEND, m);
+        const int left = tree_left<THREADS>(w, t.items + (int64_t)(base + unit) * TREE_PEND, m, t.diag);
         // The last unit of the group to finish goes on with all of its
         // subtrees; the records are written while that is being found out.
         static_assert(TREE_GROUP == 32, "one unit of a group per lane");
@@ -630,8 +639,10 @@ bh_tree_kernel(const KeyT *__restrict__ keys, TreeArgs t) {
         apart = true;
         int total = w.before[TREE_GROUP];
         // More than fit (trees far deeper than log2 n): join them piece by
-        // piece; a piece leaves fewer than half its items, which go back to
-        // the front of the same storage.
+        // piece; what a piece leaves goes back to the front of the same
+        // storage.  A full piece leaves at most TREE_PEND of TREE_CHUNK items,
+        // so every sweep leaves fewer than it took, whatever the keys.
+        static_assert(TREE_PEND < TREE_CHUNK, "a sweep ends with fewer items");
         while (total > TREE_CHUNK) {
             int out = 0;
             for (int i0 = 0; i0 < total; i0 += TREE_CHUNK) {
@@ -642,7 +653,7 @@ bh_tree_kernel(const KeyT *__restrict__ keys, TreeArgs t) {
                 tree_join<THREADS>(w, m);
                 tree_records<THREADS>(w, t, m, [&](int i) { return load_item(item(i0 + i)).s; });
                 __syncthreads();  // the items are read
-                out += tree_left<THREADS>(w, items + out, m);
+                out += tree_left<THREADS>(w, items + out, m, t.diag);
             }
             __syncthreads();
             __threadfence();
@@ -1357,6 +1368,26 @@ extern "C" int gb_sort_wait_probe(int spin_limit, int publish_first, uint32_t *e
     if (excl) cudaFree(excl);
     if (diag) cudaFree(diag);
     return rc;
+}
+
+extern "C" int gb_bh_tree_probe(gb_bh_t *h, const float *xm, const void *keys, const uint32_t *order, int64_t n,
+                                void *stream) {
+    GB_TRY(check_bh(h, n));
+    if (n < 1) return fail(GB_EINVAL, "n must be >= 1");
+    GB_TRY(check_ptr(xm, "xm"));
+    if (!keys || !order) return fail(GB_EINVAL, "NULL argument");
+    cudaStream_t s = (cudaStream_t)stream;
+    const bool groups = h->tpl == 3;
+    int64_t units, ngroups;
+    tree_units(n, &units, &ngroups);
+    GB_CUDA_TRY(cudaMemcpyAsync(h->keys[0], keys, key_size(h->key_bits) * n, cudaMemcpyDeviceToDevice, s));
+    GB_CUDA_TRY(cudaMemcpyAsync(h->vals[0], order, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, s));
+    GB_CUDA_TRY(cudaMemsetAsync(h->tree_done, 0, sizeof(unsigned) * ngroups, s));
+    if (groups) GB_CUDA_TRY(cudaMemsetAsync(h->gsize, 0, sizeof(int) * n, s));
+    if (h->key_bits == 10) GB_TRY(build_tree<uint32_t>(h, (const float4 *)xm, h->vals[0], n, groups, s));
+    else GB_TRY(build_tree<uint64_t>(h, (const float4 *)xm, h->vals[0], n, groups, s));
+    h->n = n;
+    return GB_OK;
 }
 
 extern "C" int gb_bh_set_check(gb_bh_t *h, int on) {
