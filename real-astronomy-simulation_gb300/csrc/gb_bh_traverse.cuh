@@ -114,6 +114,11 @@ constexpr int64_t WALK_4_N = 8192, WALK_8_N = 20480, WALK_16_N = 65536;
 constexpr int WALK_WARPS = 2;
 constexpr int WALK_RESERVE = 100;
 constexpr int WALK_LIST = 32;  // buffered records per warp
+// Greatest depth of an element, the 7 bits below the expanded flag.  A consistent
+// tree has 63 key bits + 31 index bits; in any other the depth stays there and
+// the bound on the rounds ends the walk.  (A branch for each of these two guards
+// took 1.3% of the walk at 1M, a minimum each takes nothing.)
+constexpr int WALK_DEPTH = 0x7F;
 template <int T>
 struct WalkShape {
     static constexpr int CAP = 512;  // list elements; the last one ends the list
@@ -313,7 +318,8 @@ bh_walk_kernel(TravArgs a, float *__restrict__ phi, int s0, int s1) {
         cnt = stop ? __ffs(stop) - 1 : 32;
         head = cnt < got ? __shfl_sync(0xffffffffu, mine, cnt) : h;
         if (lane < cnt) {
-            const float4 *rc = a.inode + 3 * (int64_t)w.ek[mine];
+            // An index that the round found out of range is still in the list, with empty masks.
+            const float4 *rc = a.inode + 3 * (int64_t)min((unsigned)w.ek[mine], (unsigned)(n - 2));
             U = __ldg(rc);
             V = __ldg(rc + 1);
             uL = w.ea[mine];
@@ -470,7 +476,7 @@ bh_walk_kernel(TravArgs a, float *__restrict__ phi, int s0, int s1) {
             if (oR) {
                 w.ek[c1] = idR - n;
                 w.ea[c1] = oR;
-                w.fl[c1] = (unsigned char)(depth + 1);
+                w.fl[c1] = (unsigned char)min(depth + 1, WALK_DEPTH);
                 w.nx[c1] = (unsigned short)link;
                 w.sf[CAP - ns + rank] = (unsigned short)c1;
                 link = c1;

@@ -1,6 +1,7 @@
 """Keys out of order, which only an expired wait of the radix sort could hand to
-the tree: the build ends, stays in bounds and counts what it drops, and the
-handle goes on to build correct trees."""
+the tree: the build ends, stays in bounds and counts what it drops, the walks
+over such a tree end and report it, and the handle goes on to build correct
+trees."""
 import importlib
 
 import numpy as np
@@ -89,3 +90,33 @@ def test_probe_checks_its_arguments(cuda_dev):
             lib_mod.call("gb_bh_tree_probe", h, *ptrs, xm.data_ptr(), n, None)
         assert e.value.status == lib_mod.GB_EINVAL
     b.close()
+
+
+@pytest.mark.parametrize("n,shape", [(3000, -1), (10000, -1), (30000, -1), (70000, -1), (3000, 3)])
+@pytest.mark.parametrize("kind", ["random", "alternating"])
+def test_walk_over_an_inconsistent_tree(cuda_dev, n, shape, kind):
+    """The nodes that were not made keep the records of the build before, of a
+    larger system: their children lie past this one's nodes, or form cycles.
+    Sizes: every group width of the walk (4, 8, 16 and 32 targets)."""
+    pkg = importlib.import_module(PKG_NAME)
+    lib_mod = importlib.import_module(PKG_NAME + "._lib")
+    bhmod = importlib.import_module(PKG_NAME + ".solvers.barnes_hut")
+    big, xm = _disk(cuda_dev, 2 * n, 4), _disk(cuda_dev, n, 5)
+    b = bhmod.BarnesHut(2 * n, theta=0.5, softening=0.05, max_stack=1 << 20, device=cuda_dev, check=True)
+    b.set_traversal(shape)
+    b.build(big)
+    _probe(b, xm, _out_of_order(kind, n, 21))
+    for phi in (None, torch.zeros(n, dtype=torch.float32, device=cuda_dev)):
+        acc = torch.zeros_like(xm)
+        b.diag(reset=True)  # the build's own count
+        with pytest.raises(pkg.GravityError, match="inconsistent tree") as e:
+            b.accel(acc, phi=phi)
+        assert e.value.status == lib_mod.GB_EINVAL
+    out, want = torch.zeros_like(big), torch.zeros_like(big)
+    b.compute(big, out)  # a checked call: raises if it counts anything
+    ref = bhmod.BarnesHut(2 * n, theta=0.5, softening=0.05, max_stack=1 << 20, device=cuda_dev, check=True)
+    ref.set_traversal(shape)
+    ref.compute(big, want)
+    assert torch.equal(out, want)
+    b.close()
+    ref.close()
