@@ -673,9 +673,10 @@ __device__ __forceinline__ void gw_group(GwWarp &w, const TravArgs &a, float *__
         }
         float4 A = make_float4(0.f, 0.f, 0.f, 0.f), B = A, C = A;
         if (act) {
-            A = __ldg(a.inode + 3 * k);      // {x_L, x_R, y_L, y_R}
-            B = __ldg(a.inode + 3 * k + 1);  // {z_L, z_R, m_L, m_R}
-            C = __ldg(a.inode + 3 * k + 2);  // {size2_L, size2_R, id_L, id_R}
+            const float4 *rec = a.inode + 3 * (int64_t)k;
+            A = __ldg(rec);      // {x_L, x_R, y_L, y_R}
+            B = __ldg(rec + 1);  // {z_L, z_R, m_L, m_R}
+            C = __ldg(rec + 2);  // {size2_L, size2_R, id_L, id_R}
         }
         if (COUNT) reads += __popc(__ballot_sync(0xffffffffu, act));
         // A leaf child carries size2 = -1 and is always accepted.
