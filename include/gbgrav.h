@@ -524,6 +524,14 @@ uint64_t gb_grid_launch_count(gb_grid_t *h);
 int gb_sort_wait_probe(int spin_limit, int publish_first, uint32_t *excl_out,
                        uint64_t *timeouts_out);
 
+/* The same for the look-back's second level, over groups of 16 tiles: tile 16
+ * of 17, of which every earlier one counts d for digit d.  publish = 0: tile 15
+ * has not published, so the sum of its group stays incomplete: GB_ETIMEOUT and
+ * *timeouts_out = 256; 1: all have, 2: only the group's inclusive prefix is
+ * there: excl_out[d] = 16 d and GB_OK. */
+int gb_sort_group_wait_probe(int spin_limit, int publish, uint32_t *excl_out,
+                             uint64_t *timeouts_out);
+
 /* Test support for the tree kernel's bounds: builds the tree of n particles
  * over the given keys (device, n uint32 for key_bits 10, n uint64 for 21) and
  * order (device, particle of each leaf) as they are, without sorting.  Keys out

@@ -127,6 +127,7 @@ SIGNATURES = {
     "gb_bh_set_graph": (I32, [P, I32]),
     "gb_bh_set_check": (I32, [P, I32]),
     "gb_sort_wait_probe": (I32, [I32, I32, P, P]),
+    "gb_sort_group_wait_probe": (I32, [I32, I32, P, P]),
     "gb_bh_tree_probe": (I32, [P, P, P, P, I64, P]),
     "gb_kick": (I32, [P, P, I64, F32, P]),
     "gb_drift": (I32, [P, P, I64, F32, P]),

@@ -1323,51 +1323,66 @@ extern "C" int gb_bh_energy(gb_bh_t *h, const float *xm, const float *vel, const
     return GB_OK;
 }
 
-// One CTA runs the radix sort's look-back for tile 1 of a two-tile status
-// array.  publish_first = 1: each thread first publishes tile 0's count
-// (its digit d), so the look-back returns d; 0: tile 0 never
-// publishes and every wait runs out after spin_limit polls.
-__global__ void sort_wait_probe_kernel(uint32_t *status, int spin_limit, int publish_first, uint32_t *excl,
+// One CTA runs the radix sort's look-back for tile t (1: the first of its
+// group's earlier tiles is tile 0; RS_GROUP: the first tile behind a whole
+// group) of a status array of t + 1 tiles, digit d in thread d; every earlier
+// tile counts d.  publish = 0: one earlier tile has not published, so every
+// wait runs out after spin_limit polls; 1: all have; 2 (t = RS_GROUP): the
+// group's inclusive prefix is there and its sum is not.
+__global__ void sort_wait_probe_kernel(uint32_t *status, int t, int spin_limit, int publish, uint32_t *excl,
                                        unsigned long long *diag) {
     const int d = threadIdx.x;
-    if (publish_first) st_relaxed_gpu(status + d, RS_AGG | (uint32_t)d);
-    const RsStatus st(status, 2);
-    rs_publish(st, 1, d, 1u);
-    excl[d] = rs_lookback(st, 1, d, 1u, spin_limit, diag);
+    const RsStatus st(status, t + 1);
+    for (int k = 0; k < (publish ? t : t - 1); ++k) rs_publish(st, k, d, (uint32_t)d);
+    if (publish == 2) {
+        rs_lookback(st, t - 1, d, (uint32_t)d, spin_limit, diag);  // publishes the group's prefix
+        st_relaxed_gpu(st.gsum + d, 0u);
+    }
+    rs_publish(st, t, d, 1u);
+    excl[d] = rs_lookback(st, t, d, 1u, spin_limit, diag);
 }
 
-extern "C" int gb_sort_wait_probe(int spin_limit, int publish_first, uint32_t *excl_out, uint64_t *timeouts_out) {
+static int sort_wait_probe(const char *call, int t, int spin_limit, int publish, uint32_t *excl_out,
+                           uint64_t *timeouts_out) {
     if (spin_limit < 1 || spin_limit > RS_SPIN_LIMIT)
         return fail(GB_EINVAL, "spin_limit must be in [1, %d] (got %d)", RS_SPIN_LIMIT, spin_limit);
     if (!excl_out || !timeouts_out) return fail(GB_EINVAL, "NULL argument");
     uint32_t *status = nullptr, *excl = nullptr;
     unsigned long long *diag = nullptr;
+    const size_t bytes = sizeof(uint32_t) * radix_status_words((int64_t)(t + 1) * RS_TILE);
     int rc = GB_OK;
-    if (cudaMalloc(&status, sizeof(uint32_t) * radix_status_words(2 * RS_TILE)) != cudaSuccess ||
-        cudaMalloc(&excl, sizeof(uint32_t) * RS_BINS) != cudaSuccess ||
+    if (cudaMalloc(&status, bytes) != cudaSuccess || cudaMalloc(&excl, sizeof(uint32_t) * RS_BINS) != cudaSuccess ||
         cudaMalloc(&diag, sizeof(unsigned long long) * DIAG_COUNT) != cudaSuccess) {
-        rc = fail(GB_ENOMEM, "gb_sort_wait_probe: device allocation failed");
+        rc = fail(GB_ENOMEM, "%s: device allocation failed", call);
     }
-    if (rc == GB_OK && (cudaMemset(status, 0, sizeof(uint32_t) * radix_status_words(2 * RS_TILE)) != cudaSuccess ||
+    if (rc == GB_OK && (cudaMemset(status, 0, bytes) != cudaSuccess ||
                         cudaMemset(diag, 0, sizeof(unsigned long long) * DIAG_COUNT) != cudaSuccess))
-        rc = fail(GB_ECUDA, "gb_sort_wait_probe: memset failed");
+        rc = fail(GB_ECUDA, "%s: memset failed", call);
     if (rc == GB_OK) {
-        sort_wait_probe_kernel<<<1, RS_BINS>>>(status, spin_limit, publish_first ? 1 : 0, excl, diag);
+        sort_wait_probe_kernel<<<1, RS_BINS>>>(status, t, spin_limit, publish, excl, diag);
         unsigned long long d[DIAG_COUNT];
         if (cudaGetLastError() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess ||
             cudaMemcpy(excl_out, excl, sizeof(uint32_t) * RS_BINS, cudaMemcpyDeviceToHost) != cudaSuccess ||
             cudaMemcpy(d, diag, sizeof(d), cudaMemcpyDeviceToHost) != cudaSuccess) {
-            rc = fail(GB_ECUDA, "gb_sort_wait_probe: %s", cudaGetErrorString(cudaGetLastError()));
+            rc = fail(GB_ECUDA, "%s: %s", call, cudaGetErrorString(cudaGetLastError()));
         } else {
             *timeouts_out = (uint64_t)d[DIAG_WAIT_TIMEOUT];
-            if (d[DIAG_WAIT_TIMEOUT])
-                rc = fail(GB_ETIMEOUT, "gb_sort_wait_probe: %llu waits expired", d[DIAG_WAIT_TIMEOUT]);
+            if (d[DIAG_WAIT_TIMEOUT]) rc = fail(GB_ETIMEOUT, "%s: %llu waits expired", call, d[DIAG_WAIT_TIMEOUT]);
         }
     }
     if (status) cudaFree(status);
     if (excl) cudaFree(excl);
     if (diag) cudaFree(diag);
     return rc;
+}
+
+extern "C" int gb_sort_wait_probe(int spin_limit, int publish_first, uint32_t *excl_out, uint64_t *timeouts_out) {
+    return sort_wait_probe("gb_sort_wait_probe", 1, spin_limit, publish_first ? 1 : 0, excl_out, timeouts_out);
+}
+
+extern "C" int gb_sort_group_wait_probe(int spin_limit, int publish, uint32_t *excl_out, uint64_t *timeouts_out) {
+    if (publish < 0 || publish > 2) return fail(GB_EINVAL, "publish must be 0, 1 or 2 (got %d)", publish);
+    return sort_wait_probe("gb_sort_group_wait_probe", RS_GROUP, spin_limit, publish, excl_out, timeouts_out);
 }
 
 extern "C" int gb_bh_tree_probe(gb_bh_t *h, const float *xm, const void *keys, const uint32_t *order, int64_t n,
