@@ -739,7 +739,13 @@ extern "C" int gb_adjoint_step(gb_direct_t *h, const float *xm, float *lx, float
         const int64_t need = max_pairs * Q * tile + max_pairs * tile + aux + 1;  // + the unit counter
         const bool counted = max_pairs * Q > slots;
         if (need * (int64_t)sizeof(float4) <= SYM_MAX_BYTES) {
-            GB_TRY(ensure_sym(h, need));
+            GB_TRY(ensure_sym(h, need, [&] {
+                int occ1 = 0;
+                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ1, adjoint_vjp_sym2_kernel<1, SYM2_T>,
+                                                              SYM2_WARPS<SYM2_T> * 32, 0);
+                return sym_most(n, h->sym_band, SYM2_T, (int64_t)h->sms * std::max(occ1, 1), 16 / SYM2_WARPS<SYM2_T>,
+                                SYM2_SMALL_T, SYM2_SMALL_Q, SYM2_SMALL_N, 1);
+            }));
             Sym2Args a;
             a.xm = (const float4 *)xm;
             a.lv = (const float4 *)lv;
@@ -798,7 +804,7 @@ extern "C" int gb_adjoint_step(gb_direct_t *h, const float *xm, float *lx, float
         const int64_t P = std::max<int64_t>(1, std::min<int64_t>((int64_t)h->sms * std::max(occs, 1), NP));
         const int64_t need = (nt + P) * SYM_T + NP * SYM_T;
         if (need * (int64_t)sizeof(float4) <= SYM_MAX_BYTES) {
-            GB_TRY(ensure_sym(h, need));
+            GB_TRY(ensure_sym(h, need, [&] { return need; }));
             SymArgs a;
             a.xm = (const float4 *)xm;
             a.lv = (const float4 *)lv;

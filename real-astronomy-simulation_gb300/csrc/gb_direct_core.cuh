@@ -223,16 +223,51 @@ struct gb_direct {
 
 namespace gb {
 
+// Source slices per tile pair (at most qmax) for a pass of the given
+// tile-pair count over `slots` resident CTAs.
+int direct_sym_slices(int64_t pairs, int64_t slots, int qmax);
+
+// Tile-pair scratch, in float4s, of the largest use below SYM_MAX_BYTES among
+// systems of up to n particles: in tiles of `tile` with the slices of
+// direct_sym_slices, or up to small_n particles in tiles of `small` with small_q
+// slices; aux: running sums per particle of a pass in bands.  Fewer particles
+// can need more: they get smaller tiles or more slices.
+inline int64_t sym_most(int64_t n, int64_t band, int tile, int64_t slots, int qmax, int small, int small_q,
+                        int64_t small_n, int aux) {
+    int64_t most = 0;
+    for (int64_t t = (n + tile - 1) / tile; t > 0; --t) {
+        const int64_t pairs = t * (t + 1) / 2;
+        const int Q = direct_sym_slices(pairs, slots, qmax);
+        const int64_t slot = (int64_t)tile * (Q + 1), budget = band / ((int64_t)sizeof(float4) * slot);
+        const int64_t need = std::min(pairs, std::max(budget, t)) * slot + (pairs > budget ? aux * t * tile : 0) + 1;
+        if (need * (int64_t)sizeof(float4) <= SYM_MAX_BYTES) most = std::max(most, need);
+    }
+    int64_t m = std::min(n, small_n);
+    while (m > 0 && !sym_one_band(m, small, small_q, band)) m -= small;
+    const int64_t t = (std::max<int64_t>(m, 0) + small - 1) / small;
+    return std::max(most, t * (t + 1) / 2 * small * (small_q + 1) + 1);
+}
+
 // Grows the handle's tile-pair scratch (shared by the symmetric force pass
-// and the symmetric adjoint, which run in stream order) to need float4s.
-inline int ensure_sym(gb_direct *h, int64_t need) {
+// and the symmetric adjoint, which run in stream order) to need float4s, and to
+// what any smaller system needs (sym_most) if there is room: a call after one
+// with more particles then allocates nothing, and a caller's graph captured over
+// the larger system keeps its scratch.
+template <typename F>
+inline int ensure_sym(gb_direct *h, int64_t need, F most) {
     if (need <= h->sym_cap) return GB_OK;
     if (h->sym) cudaFree(h->sym);
     h->sym = nullptr;
     h->sym_cap = 0;
-    if (cudaMalloc(&h->sym, sizeof(float4) * need) != cudaSuccess)
+    int64_t size = std::max(need, (int64_t)most());
+    if (size > need && cudaMalloc(&h->sym, sizeof(float4) * size) != cudaSuccess) {
+        cudaGetLastError();
+        h->sym = nullptr;
+        size = need;
+    }
+    if (!h->sym && cudaMalloc(&h->sym, sizeof(float4) * size) != cudaSuccess)
         return fail(GB_ENOMEM, "tile-pair scratch (%lld bytes)", (long long)(need * 16));
-    h->sym_cap = need;
+    h->sym_cap = size;
     return GB_OK;
 }
 
@@ -260,10 +295,8 @@ struct SymBatch {
     int64_t NU, NPtot, nfb, P;
     float4 *scratch;
 };
-// Source slices per tile pair (at most qmax) for a pass of the given
-// tile-pair count over `slots` resident CTAs, and the symmetric force
-// kernel's resident CTAs and slices for such a pass.
-int direct_sym_slices(int64_t pairs, int64_t slots, int qmax);
+// The symmetric force kernel's resident CTAs and its slices for a pass of the
+// given tile-pair count.
 struct SymShape {
     int Q;
     int64_t slots;

@@ -548,10 +548,16 @@ static DsPlan ds_plan(const gb_direct *h, int64_t n) {
     return p;
 }
 
+static int ds_scratch(gb_direct *h, const DsPlan &p, int64_t n) {
+    return ensure_sym(h, p.need, [&] {
+        return sym_most(n, h->sym_band, DS_T, p.slots, DsShape<DS_H, DS_T>::QMAX, DS_SMALL_T, DS_SMALL_Q, DS_SMALL_N, 2);
+    });
+}
+
 int reserve_direct_sym(gb_direct *h, int64_t n) {
     const DsPlan p = ds_plan(h, n);
     if (p.need * (int64_t)sizeof(float4) > SYM_MAX_BYTES) return GB_OK;
-    return ensure_sym(h, p.need);
+    return ds_scratch(h, p, n);
 }
 
 int run_direct_sym(gb_direct *h, int mode, const float4 *xm, float4 *vel, float4 *acc, float *phi, int64_t n,
@@ -559,7 +565,7 @@ int run_direct_sym(gb_direct *h, int mode, const float4 *xm, float4 *vel, float4
     *done = false;
     const DsPlan pl = ds_plan(h, n);
     if (pl.need * (int64_t)sizeof(float4) > SYM_MAX_BYTES) return GB_OK;
-    GB_TRY(ensure_sym(h, pl.need));
+    GB_TRY(ds_scratch(h, pl, n));
     DsArgs a{};
     a.xm = xm;
     a.vel = vel;
