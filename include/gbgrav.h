@@ -297,9 +297,10 @@ int gb_bh_diag(gb_bh_t *h, gb_diag_t *out, int reset);
 
 /* Traversal shape.  -1 (default), 0, 1 and 2: the per-particle walk, in which
  * each target accepts exactly the reference's node set (4 to 32
- * key-consecutive targets share a warp, by n).  The four values run the same
- * kernel and give bit-identical results; 0 to 2 named kernels of their own
- * once and stay accepted.
+ * key-consecutive targets share a warp, by n; for large theta one node at a
+ * time, per target or per warp).  The kernel depends on n and theta, not on
+ * which of the four values is set, and the results on neither; 0 to 2 named
+ * kernels of their own once and stay accepted.
  * 3 (opt-in): group walk.  The targets are cut into groups, the largest
  * subtrees with at most 32 leaves; a group accepts a node when
  * size^2 < theta^2 (dmin^2 + eps^2), dmin the distance from the node's

@@ -17,7 +17,8 @@
 //               and the result is independent of scheduling (:124-177 use
 //               FP64 atomics on every ancestor instead)
 //   4 traverse  per-particle walk: 4 to 32 key-consecutive targets share a
-//               warp and its list of opened nodes; every target applies the reference's own acceptance
+//               warp and its list of opened nodes (for large theta one node
+//               at a time); every target applies the reference's own acceptance
 //               test size^2 < theta^2 (r^2 + eps^2) (:204-210), so each
 //               particle accepts exactly the node set of _traverse
 //               (:180-217); the max_stack rule (:212) is kept and the skipped
@@ -1026,6 +1027,21 @@ struct GroupLaunch {
     }
 };
 template <bool KDK, bool COUNT, bool PHI>
+struct ShortWalkLaunch {
+    static void go(WalkForm form, int2 r, const TravArgs *a, float *phi, cudaStream_t s) {
+        const int64_t nt = (int64_t)r.y - r.x;
+        if (form == WALK_WARP) {
+            constexpr int T = WARP_WALK_WARPS * 32;
+            bh_warp_walk_kernel<KDK, COUNT, PHI><<<(unsigned)((nt + T - 1) / T), T, 0, s>>>(*a, phi, r.x, r.y);
+        } else {
+            constexpr int T = LANE_WALK_THREADS;
+            const int room = std::min(a->max_stack, LANE_WALK_STACK);
+            bh_lane_walk_kernel<KDK, COUNT, PHI>
+                <<<(unsigned)((nt + T - 1) / T), T, sizeof(unsigned) * room * T, s>>>(*a, phi, r.x, r.y, room);
+        }
+    }
+};
+template <bool KDK, bool COUNT, bool PHI>
 struct WalkLaunch {
     template <int T>
     static void run(int2 r, const TravArgs *a, float *phi, cudaStream_t s) {
@@ -1085,6 +1101,8 @@ static int traverse(gb_bh_t *h, float4 *acc, float4 *vel, float *phi, float thet
             else GB_TRY(build_tree<uint64_t>(h, nullptr, nullptr, n, true, s));
         }
         dispatch3<GroupLaunch>(kdk, count, phi != nullptr, grid, &a, (const int *)h->gsize, phi, range, s);
+    } else if (const WalkForm form = walk_form(n, theta); form != WALK_ROUNDS) {
+        dispatch3<ShortWalkLaunch>(kdk, count, phi != nullptr, form, range, &a, phi, s);
     } else {
         const int group = n < WALK_4_N ? 4 : n < WALK_8_N ? 8 : n < WALK_16_N ? 16 : 32;
         dispatch3<WalkLaunch>(kdk, count, phi != nullptr, group, range, &a, phi, s);

@@ -4,6 +4,9 @@
 //                    each particle accepts exactly the node set of the
 //                    reference's _traverse (core/solvers/barnes_hut.py:
 //                    180-217)
+//   bh_lane_walk_kernel, bh_warp_walk_kernel
+//                    the same walk, one node at a time, for large opening
+//                    angles, with the same results
 //   bh_group_kernel  the opt-in group walk (a refinement of each target's
 //                    node set, one walk per leaf group)
 // Node records: inode[3k .. 3k+2] = the two children of internal node k as
@@ -535,6 +538,290 @@ bh_walk_kernel(TravArgs a, float *__restrict__ phi, int s0, int s1) {
     if (p >= (uint32_t)n) return;
     if (PHI) phi[p] = pw;
     trav_write<KDK>(a, p, px, py, pz, ax + tx, ay + ty, az + tz);
+}
+
+// ------------------------------------------------------------- short walks
+// Large opening angles make short walks: most of the rounds of bh_walk_kernel go
+// down the tree towards the targets with few nodes each, at the price of 32.
+// These two kernels expand one node at a time, per warp or per lane, and add
+// every accepted child where they meet it.  Right subtrees come first, so each
+// target sums the same nodes in the same order as in bh_walk_kernel, bit for bit.
+//
+// Walk time over that of bh_walk_kernel (disk, Plummer sphere, uniform cube; eps
+// 0.05; 63-bit keys), per lane at theta 1.0 / 1.1 / 1.2 / 1.3 (15,000 and 22,000,
+// theta 1.4: 0.94 1.20 0.79, 0.89 1.12 0.77):
+//   25,000: 1.43 1.90 1.35 / 1.20 1.59 1.03 / 1.05 1.36 0.91 / 0.90 1.17 0.82
+//   40,000: 1.26 1.69 1.17 / 1.11 1.41 0.84 / 1.03 1.19 0.79 / 0.87 1.08 0.68
+//   50,000: 1.23 1.42 1.00 / 1.06 1.18 0.78 / 0.93 0.95 0.69 / 0.79 0.85 0.58
+//   85,000: 0.94 1.20 0.88 / 0.83 0.97 0.65 / 0.71 0.81 0.60 / 0.63 0.71 0.53
+//  100,000: 0.92 1.10 0.75 / 0.77 0.94 0.53 / 0.64 0.79 0.50 / 0.57 0.68 0.44
+// and per warp at theta 0.8 / 0.9 / 1.0 / 1.2:
+//  131,072: 1.35 1.15 1.17 / 1.23 1.08 0.97 / 1.10 0.96 0.80 / 0.81 0.74 0.59
+//  250,000: 1.22 1.23 1.08 / 1.11 1.12 0.88 / 1.00 0.97 0.70 / 0.74 0.72 0.49
+//  500,000: 1.10 1.07 0.94 / 0.98 0.97 0.74 / 0.85 0.84 0.57 / 0.64 0.61 0.38
+//  1.5M:    1.01 1.04 0.79 / 0.90 0.92 0.60 / 0.77 0.79 0.46 / 0.57 0.59 0.31
+//  4M:      1.01 1.02 0.72 / 0.89 0.91 0.54 / 0.76 0.77 0.41 / 0.54 0.58 0.29
+// (100,000, theta 1.2: 96 us in rounds, 62 per lane, 82 per warp on the disk; 1M:
+// 813 in rounds, 473 per warp.)  Per lane is the faster of the two up to about
+// 120,000 (100,000: see above; 131,072, theta 1.2: 0.71 0.96 0.63).  The lines of
+// walk_form lie where the geometric mean of the three crosses 1.
+enum WalkForm { WALK_ROUNDS, WALK_LANE, WALK_WARP };
+static inline WalkForm walk_form(int64_t n, float theta) {
+    if (n < 12000) return WALK_ROUNDS;
+    if (n < 131072) {
+        const float line = n < 25000 ? 1.4f : n < 40000 ? 1.3f : n < 50000 ? 1.2f : n < 85000 ? 1.1f : 1.0f;
+        return theta >= line ? WALK_LANE : WALK_ROUNDS;
+    }
+    const float line = n < 150000 ? 1.0f : n < 300000 ? 0.95f : n < 500000 ? 0.9f : n < 1200000 ? 0.85f : 0.8f;
+    return theta >= line ? WALK_WARP : WALK_ROUNDS;
+}
+
+// One lane's target s and its sums.
+struct OneWalk {
+    float px, py, pz, pm;
+    f2 PX, PY, PZ;
+    float ax, ay, az, aw;  // the root's term
+    WalkSum sum;           // over the (left, right) children
+    unsigned n_int, n_test, drops;
+    bool self;             // met the target's own leaf
+};
+
+__device__ __forceinline__ OneWalk one_target(const TravArgs &a, int s, bool valid) {
+    OneWalk w;
+    const float4 p = valid ? __ldg(a.leaf + s) : make_float4(0.f, 0.f, 0.f, 0.f);
+    w.px = p.x; w.py = p.y; w.pz = p.z; w.pm = p.w;
+    w.PX = pack2(p.x, p.x);
+    w.PY = pack2(p.y, p.y);
+    w.PZ = pack2(p.z, p.z);
+    w.ax = w.ay = w.az = w.aw = 0.f;
+    w.sum.X = w.sum.Y = w.sum.Z = w.sum.W = 0ull;
+    w.n_int = w.n_test = w.drops = 0;
+    w.self = false;
+    return w;
+}
+
+// Whether a target that opens a node popped at `depth` may push its children (:212).
+__device__ __forceinline__ bool one_room(OneWalk &w, bool open, int depth, int max_stack) {
+    if (depth + 2 <= max_stack) return open;
+    w.drops += open ? 1u : 0u;
+    return false;
+}
+
+// The root, popped first with an empty stack; returns whether it is opened.
+__device__ __forceinline__ bool one_root(OneWalk &w, const TravArgs &a, bool valid) {
+    const float4 R0 = __ldg(a.root), R1 = __ldg(a.root + 1);
+    const float dx = R0.x - w.px, dy = R0.y - w.py, dz = R0.z - w.pz;
+    const float r2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmaf_rn(dx, dx, a.eps2)));
+    const bool acc = valid && R1.x < a.theta2 * r2;
+    if (acc) {
+        const float inv = rsqrt_approx(r2);
+        const float sc = R0.w * inv * inv * inv;
+        w.ax = __fmul_rn(sc, dx);
+        w.ay = __fmul_rn(sc, dy);
+        w.az = __fmul_rn(sc, dz);
+        w.aw = R0.w * inv;
+        w.n_int = 1;
+    }
+    w.n_test = valid ? 1 : 0;
+    return one_room(w, valid && !acc, 0, a.max_stack);
+}
+
+// Both children of record {A, B, C} for the lane's target, when `in`: accepted
+// ones are added, and the ones to open returned.
+template <bool COUNT, bool PHI>
+__device__ __forceinline__ void one_pair(OneWalk &w, const TravArgs &a, ulonglong2 A, ulonglong2 B, float4 C, int s,
+                                         bool in, f2 E2, f2 TH2, bool &openL, bool &openR) {
+    const f2 dx = sub2(A.x, w.PX), dy = sub2(A.y, w.PY), dz = sub2(B.x, w.PZ);
+    f2 r2 = fma2(dx, dx, E2);
+    r2 = fma2(dy, dy, r2);
+    r2 = fma2(dz, dz, r2);
+    float tL, tR, cL, cR;
+    unpack2(mul2(TH2, r2), tL, tR);
+    const bool accL = in && C.x < tL, accR = in && C.y < tR;
+    const f2 inv = rsqrt2(r2);
+    unpack2(mul2(mul2(B.y, inv), mul2(inv, inv)), cL, cR);
+    const f2 sc = pack2(accL ? cL : 0.f, accR ? cR : 0.f);
+    w.sum.X = fma2(sc, dx, w.sum.X);
+    w.sum.Y = fma2(sc, dy, w.sum.Y);
+    w.sum.Z = fma2(sc, dz, w.sum.Z);
+    if (PHI) w.sum.W = fma2(sc, r2, w.sum.W);
+    if (PHI || COUNT) {
+        const bool ownL = __float_as_int(C.z) == s, ownR = __float_as_int(C.w) == s;
+        if (PHI) w.self |= (accL && ownL) || (accR && ownR);
+        if (COUNT) {
+            w.n_int += (accL && !ownL ? 1u : 0u) + (accR && !ownR ? 1u : 0u);
+            w.n_test += (in && C.x >= 0.f ? 1u : 0u) + (in && C.y >= 0.f ? 1u : 0u);
+        }
+    }
+    openL = in && !accL;
+    openR = in && !accR;
+}
+
+// The warp's counters, and the lane's target written.  reads, roots: records
+// read by the lane or its warp.
+template <bool KDK, bool COUNT, bool PHI>
+__device__ __forceinline__ void one_write(OneWalk &w, const TravArgs &a, float *__restrict__ phi, int s, bool valid,
+                                          unsigned bad, unsigned reads, unsigned roots) {
+    const int lane = threadIdx.x & 31;
+    const unsigned dsum = __reduce_add_sync(0xffffffffu, w.drops), bsum = __reduce_add_sync(0xffffffffu, bad);
+    if (lane == 0) {
+        if (dsum) atomicAdd(a.diag + DIAG_STACK_DROPS, (unsigned long long)dsum);
+        if (bsum) atomicAdd(a.diag + DIAG_BAD_TREE, (unsigned long long)bsum);
+    }
+    if (COUNT) {
+        const unsigned isum = __reduce_add_sync(0xffffffffu, w.n_int), tsum = __reduce_add_sync(0xffffffffu, w.n_test);
+        const unsigned rsum = __reduce_add_sync(0xffffffffu, reads), osum = __reduce_add_sync(0xffffffffu, roots);
+        if (lane == 0) {
+            atomicAdd(a.diag + DIAG_NODE_READS, (unsigned long long)rsum);
+            atomicAdd(a.diag + DIAG_ROOT_READS, (unsigned long long)osum);
+            atomicAdd(a.diag + DIAG_INTERACTIONS, (unsigned long long)isum);
+            atomicAdd(a.diag + DIAG_TESTS, (unsigned long long)tsum);
+        }
+    }
+    if (!valid) return;
+    const uint32_t p = __ldg(a.order + s);
+    if (p >= (uint32_t)a.n) return;
+    float xl, xr, yl, yr, zl, zr;
+    unpack2(w.sum.X, xl, xr);
+    unpack2(w.sum.Y, yl, yr);
+    unpack2(w.sum.Z, zl, zr);
+    if (PHI) {  // the children's terms include the target's own leaf: remove it
+        float wl, wr;
+        unpack2(w.sum.W, wl, wr);
+        float pw = w.aw + (wl + wr);
+        if (w.self) {
+            const float inv = rsqrt_approx(a.eps2);
+            pw = __fmaf_rn(-((w.pm * inv) * (inv * inv)), a.eps2, pw);
+        }
+        phi[p] = pw;
+    }
+    trav_write<KDK>(a, p, w.px, w.py, w.pz, w.ax + (xl + xr), w.ay + (yl + yr), w.az + (zl + zr));
+}
+
+// Per warp: 32 key-consecutive targets share a stack of {node, mask of the
+// targets that opened it, depth}.
+constexpr int WARP_WALK_WARPS = 4;
+constexpr int WARP_WALK_STACK = 128;  // one pending left child per level of right turns: 94 in a consistent tree
+
+template <bool KDK, bool COUNT, bool PHI>
+__global__ void __launch_bounds__(WARP_WALK_WARPS * 32)
+bh_warp_walk_kernel(TravArgs a, float *__restrict__ phi, int s0, int s1) {
+    __shared__ int4 stk[WARP_WALK_WARPS][WARP_WALK_STACK];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, n = a.n;
+    const int g0 = s0 + (blockIdx.x * WARP_WALK_WARPS + wid) * 32, s = g0 + lane;
+    if (g0 >= s1) return;  // whole warp out of range
+    const bool valid = s < s1;
+    OneWalk w = one_target(a, s, valid);
+    const f2 E2 = pack2(a.eps2, a.eps2), TH2 = pack2(a.theta2, a.theta2);
+    unsigned bad = 0, reads = 0, m = 0;
+    int top = 0, k = 0, depth = 0;
+    if (n >= 2) m = __ballot_sync(0xffffffffu, one_root(w, a, valid));
+    // A consistent tree expands each internal node at most once per warp, so
+    // more than n - 1 nodes mean a corrupted tree.
+    for (int left = n; m;) {
+        unsigned mL = 0, mR = 0;
+        int idL = 0, idR = 0;
+        if (--left < 0 || (unsigned)k >= (unsigned)(n - 1)) {  // never for a consistent tree
+            bad += (m >> lane) & 1u;
+        } else {
+            const float4 *rec = a.inode + 3 * (int64_t)k;
+            const ulonglong2 A = __ldg(reinterpret_cast<const ulonglong2 *>(rec));
+            const ulonglong2 B = __ldg(reinterpret_cast<const ulonglong2 *>(rec + 1));
+            const float4 C = __ldg(rec + 2);
+            idL = __float_as_int(C.z);
+            idR = __float_as_int(C.w);
+            reads += lane == 0 ? 1u : 0u;
+            bool openL, openR;
+            one_pair<COUNT, PHI>(w, a, A, B, C, s, (m >> lane) & 1u, E2, TH2, openL, openR);
+            if (depth + 3 > a.max_stack) {  // the rule only bites near max_stack
+                openR = one_room(w, openR, depth + 1, a.max_stack);
+                openL = one_room(w, openL, depth, a.max_stack);
+            }
+            mL = __ballot_sync(0xffffffffu, openL);
+            mR = __ballot_sync(0xffffffffu, openR);
+        }
+        if (mR) {  // the right child next; a left child waits on the stack
+            if (mL) {
+                if (top < WARP_WALK_STACK) stk[wid][top++] = make_int4(idL - n, (int)mL, depth, 0);
+            }
+            k = idR - n;
+            m = mR;
+            ++depth;
+        } else if (mL) {
+            k = idL - n;
+            m = mL;
+        } else if (top > 0) {
+            __syncwarp();
+            const int4 e = stk[wid][--top];
+            __syncwarp();
+            k = e.x;
+            m = (unsigned)e.y;
+            depth = e.z;
+        } else {
+            m = 0;
+        }
+    }
+    one_write<KDK, COUNT, PHI>(w, a, phi, s, valid, bad, reads, lane == 0 ? 1u : 0u);
+}
+
+// Per lane: every lane walks for its own target, its pending left children as
+// {node, 25 bits; depth, 7 bits} on a stack of its own, laid out so that lanes
+// meet no bank conflicts whatever their depth.
+constexpr int LANE_WALK_THREADS = 128;
+constexpr int LANE_WALK_BITS = 25;
+constexpr int LANE_WALK_STACK = 96;  // one pending left child per level of right turns (94)
+
+template <bool KDK, bool COUNT, bool PHI>
+__global__ void __launch_bounds__(LANE_WALK_THREADS)
+bh_lane_walk_kernel(TravArgs a, float *__restrict__ phi, int s0, int s1, int room) {
+    extern __shared__ unsigned lane_stk[];  // [room][LANE_WALK_THREADS]
+    const int tid = threadIdx.x, n = a.n, s = s0 + blockIdx.x * LANE_WALK_THREADS + tid;
+    const bool valid = s < s1;
+    OneWalk w = one_target(a, s, valid);
+    const f2 E2 = pack2(a.eps2, a.eps2), TH2 = pack2(a.theta2, a.theta2);
+    unsigned bad = 0, reads = 0;
+    int k = 0, depth = 0, top = 0;
+    bool active = n >= 2 && one_root(w, a, valid);
+    for (int left = n;;) {
+        if (!active) {
+            if (top == 0) break;
+            const unsigned e = lane_stk[--top * LANE_WALK_THREADS + tid];
+            k = (int)(e & ((1u << LANE_WALK_BITS) - 1u));
+            depth = (int)(e >> LANE_WALK_BITS);
+            active = true;
+        }
+        if (--left < 0 || (unsigned)k >= (unsigned)(n - 1)) {  // never for a consistent tree
+            ++bad;
+            break;
+        }
+        const float4 *rec = a.inode + 3 * (int64_t)k;
+        const ulonglong2 A = __ldg(reinterpret_cast<const ulonglong2 *>(rec));
+        const ulonglong2 B = __ldg(reinterpret_cast<const ulonglong2 *>(rec + 1));
+        const float4 C = __ldg(rec + 2);
+        const int idL = __float_as_int(C.z), idR = __float_as_int(C.w);
+        if (COUNT) ++reads;
+        bool openL, openR;
+        one_pair<COUNT, PHI>(w, a, A, B, C, s, true, E2, TH2, openL, openR);
+        if (depth + 3 > a.max_stack) {
+            openR = one_room(w, openR, depth + 1, a.max_stack);
+            openL = one_room(w, openL, depth, a.max_stack);
+        }
+        if (openR) {
+            if (openL) {
+                if (top < room) lane_stk[top++ * LANE_WALK_THREADS + tid] =
+                    (unsigned)(idL - n) | (unsigned)depth << LANE_WALK_BITS;
+                else ++bad;  // never for a consistent tree
+            }
+            k = idR - n;
+            ++depth;
+        } else if (openL) {
+            k = idL - n;
+        } else {
+            active = false;
+        }
+    }
+    __syncwarp();
+    one_write<KDK, COUNT, PHI>(w, a, phi, s, valid, bad, reads, n >= 2 && valid ? 1u : 0u);
 }
 
 // ------------------------------------------------------------- group walk

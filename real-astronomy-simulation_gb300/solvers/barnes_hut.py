@@ -185,8 +185,8 @@ class BarnesHut:
 
     def set_traversal(self, targets_per_lane: int) -> None:
         """Traversal shape: -1 (default), 0, 1 or 2: the per-particle walk;
-        results are bit-identical across these values, which run the same
-        kernel.  3 (opt-in): group walk, each group of up to 32
+        the kernel is picked by n and theta, and results are bit-identical
+        across these values.  3 (opt-in): group walk, each group of up to 32
         key-consecutive targets (one subtree) shares the node set its
         bounding box accepts under the reference's test: every target sums
         a refinement of its own node set, so the error is no larger, but

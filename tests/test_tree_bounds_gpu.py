@@ -92,17 +92,19 @@ def test_probe_checks_its_arguments(cuda_dev):
     b.close()
 
 
-@pytest.mark.parametrize("n,shape", [(3000, -1), (10000, -1), (30000, -1), (70000, -1), (3000, 3)])
+@pytest.mark.parametrize("n,shape,theta", [(3000, -1, 0.5), (10000, -1, 0.5), (30000, -1, 0.5), (70000, -1, 0.5),
+                                           (3000, 3, 0.5), (30000, -1, 1.3), (140000, -1, 1.0)])
 @pytest.mark.parametrize("kind", ["random", "alternating"])
-def test_walk_over_an_inconsistent_tree(cuda_dev, n, shape, kind):
+def test_walk_over_an_inconsistent_tree(cuda_dev, n, shape, theta, kind):
     """The nodes that were not made keep the records of the build before, of a
     larger system: their children lie past this one's nodes, or form cycles.
-    Sizes: every group width of the walk (4, 8, 16 and 32 targets)."""
+    Sizes: every group width of the walk in rounds (4, 8, 16 and 32 targets), the
+    group walk, and the walks per lane and per warp."""
     pkg = importlib.import_module(PKG_NAME)
     lib_mod = importlib.import_module(PKG_NAME + "._lib")
     bhmod = importlib.import_module(PKG_NAME + ".solvers.barnes_hut")
     big, xm = _disk(cuda_dev, 2 * n, 4), _disk(cuda_dev, n, 5)
-    b = bhmod.BarnesHut(2 * n, theta=0.5, softening=0.05, max_stack=1 << 20, device=cuda_dev, check=True)
+    b = bhmod.BarnesHut(2 * n, theta=theta, softening=0.05, max_stack=1 << 20, device=cuda_dev, check=True)
     b.set_traversal(shape)
     b.build(big)
     _probe(b, xm, _out_of_order(kind, n, 21))
@@ -114,7 +116,7 @@ def test_walk_over_an_inconsistent_tree(cuda_dev, n, shape, kind):
         assert e.value.status == lib_mod.GB_EINVAL
     out, want = torch.zeros_like(big), torch.zeros_like(big)
     b.compute(big, out)  # a checked call: raises if it counts anything
-    ref = bhmod.BarnesHut(2 * n, theta=0.5, softening=0.05, max_stack=1 << 20, device=cuda_dev, check=True)
+    ref = bhmod.BarnesHut(2 * n, theta=theta, softening=0.05, max_stack=1 << 20, device=cuda_dev, check=True)
     ref.set_traversal(shape)
     ref.compute(big, want)
     assert torch.equal(out, want)
