@@ -480,8 +480,10 @@ __device__ __forceinline__ void sym2_round(const float4 *__restrict__ sxm, const
 template <int Q, int TILE>
 __global__ void __launch_bounds__(SYM2_WARPS<TILE> * 32, 16 / SYM2_WARPS<TILE>) adjoint_vjp_sym2_kernel(Sym2Args a) {
     constexpr int WARPS = SYM2_WARPS<TILE>, G = TILE / 32 / Q, SPAN = G * 32;
-    // Steps unrolled: 4,096 particles 26.7 us with 2, 25.4 with 3; 65,536: 2.94 ms, 3.01.
-    constexpr int UNROLL = TILE == SYM2_SMALL_T ? 3 : 2;
+    // Steps unrolled, 2 / 3: 4,096 particles 26.7 / 25.4 us; 65,536 (two slices): 2.94
+    // / 3.01 ms; in one slice 72,000: 3.65 / 3.56 ms, 80,000: 4.51 / 4.43, 130,000:
+    // 11.60 / 11.48.
+    constexpr int UNROLL = TILE == SYM2_SMALL_T || Q == 1 ? 3 : 2;
     static_assert(G >= WARPS, "each warp of a round takes its own source group");
     __shared__ float4 sxm[TILE], sw[TILE], sacc[TILE];
     __shared__ long long s_unit;
