@@ -318,7 +318,9 @@ int gb_bh_set_traversal(gb_bh_t *h, int targets_per_lane);
 /* Stage timing for measurement: with timing enabled, every build/step records
  * CUDA events on its stream at the boundaries of the GB_BH_STAGES stages
  * (0 bbox+keys, 1 sort, 2 tree with its summaries, 3 empty since the tree and
- * its summaries are one kernel, 4 traversal).
+ * its summaries are one kernel, 4 traversal; up to 262,144 particles, 131,072
+ * with key_bits 10, the sort's first kernel makes the keys, so that they count
+ * in stage 1 and stage 0 is the box).
  * gb_bh_stage_times synchronises, returns the summed milliseconds per stage
  * over the (at most GB_BH_TIMING_STEPS) steps since the last call, and the
  * step count.  gb_bh_launch_count returns the kernels this handle launched.

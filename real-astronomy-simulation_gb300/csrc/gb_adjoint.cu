@@ -367,9 +367,9 @@ constexpr int SYM2_WARPS = TILE / 128;
 // Small systems (at most SYM2_SMALL_N particles): tiles of 256, two warps, four
 // source slices per tile pair.  As in the force pass the time is one unit's
 // length while the units fit one wave, and half of it here.  Microseconds per
-// VJP, tiles of 512 / 256: 1,000: 20.3 / 10.2; 4,096: 20.7 / 18.7; 6,144:
-// 47.8 / 32.4; 8,000: 60.9 / 53.6; beyond that the second wave's share falls
-// and the slots of the larger tiles are half as many.
+// VJP with its fix-up, tiles of 512 / 256: 1,000: 21.4 / 13.2; 4,096: 22.3 / 20.5;
+// 6,144: 48.7 / 34.7; 8,000: 63.0 / 60.6 (10,000: 94.3 / 88.2, so the line could
+// lie a little higher).
 constexpr int SYM2_SMALL_T = 256, SYM2_SMALL_Q = 4;
 constexpr int64_t SYM2_SMALL_N = 8192;
 

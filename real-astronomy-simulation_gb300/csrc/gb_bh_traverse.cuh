@@ -1033,7 +1033,7 @@ __device__ __forceinline__ void gw_group(GwWarp &w, const TravArgs &a, float *__
 }
 
 // Warp w walks the groups whose first leaf lies in [32 w, 32 w + 32) (gsize
-// from the Karras kernel), one after the other.
+// from bh_tree_kernel), one after the other.
 // 32 resident warps per SM (64 registers, 13 KB of shared memory per CTA of
 // 2 warps): 7.8% less time than 24 warps on the 1M disk; CTAs of 2 warps
 // against 4: 1.3% less (a CTA retires when its slowest warp is done).

@@ -57,9 +57,11 @@ constexpr int DS_H = 4;
 // sources x 8 targets a lane, one of 256 for 64 x 4.  Up to 6,144 particles
 // (300 tile pairs, 1,200 units) the small units still run in one wave, so each
 // CTA takes the unit of its index and the counter with its memset is left out.
-// Microseconds per KDK step, tiles of 512 with the counter / 512 without / 256:
-// 1,000: 18.5 / 14.7 / 10.6; 4,096: 18.5 / 15.7 / 12.9; 6,144: - / 26.2 / 19.8;
-// past the wave the twice as many slots cost more: 8,000: - / 32.9 / 37.2.
+// Microseconds per KDK step on the device (graphs of 8 steps), tiles of 512 / 256:
+// 1,000: 13.8 / 8.7; 4,096: 14.8 / 12.8; 6,144: 25.6 / 19.7; past the wave the
+// twice as many slots cost more: 8,000: 32.0 / 36.9.  The counter with its memset
+// cost 512 tiles about 4 more below 6,000 (1,000: 18.5 against 14.7).  A call
+// of one step does not show this: at 1,000 it is bound by the host.
 constexpr int DS_SMALL_T = 256, DS_SMALL_H = 2, DS_SMALL_Q = 4;
 constexpr int64_t DS_SMALL_N = 6144;
 
